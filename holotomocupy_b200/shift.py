@@ -84,12 +84,14 @@ class Shift:
     def coeff(self, psi):
         """B-spline prefilter ifft2(fft2(psi) * ifB3) (shift.py:74-82)."""
         _lib.require_cuda(psi, "psi")
-        x = psi.to(torch.complex64).contiguous()
+        real = self.obj_dtype == "float32"
+        if real:   # the filter is real: the real part of its output is the filtered real part
+            x = (psi.real if psi.is_complex() else psi).to(torch.float32).contiguous()
+        else:
+            x = psi.to(torch.complex64).contiguous()
         out = torch.empty_like(x)
         b = x.numel() // (self.nzpsi * self.npsi)
-        self._call("ht_shift_coeff", self._hc, _lib.ptr(x), _lib.ptr(out), b)
-        if self.obj_dtype == "float32":
-            out = out.real.contiguous()
+        self._call("ht_shift_coeff_real" if real else "ht_shift_coeff", self._hc, _lib.ptr(x), _lib.ptr(out), b)
         return out
 
     def S(self, c, r, m):
@@ -143,21 +145,25 @@ class Shift:
         when m holds several)."""
         _lib.require_cuda(psi, "psi")
         m = float(np.asarray(m.cpu() if isinstance(m, torch.Tensor) else m, dtype=np.float64).reshape(-1)[0])
-        x = np.linspace(-1 / 2, 1 / 2 - 1 / self.npsi, self.npsi).astype("float32")
-        y = np.linspace(-1 / 2, 1 / 2 - 1 / self.nzpsi, self.nzpsi).astype("float32")
+        x = psi.to(torch.complex64).contiguous()
+        out = torch.empty_like(x)
+        b = x.numel() // (self.nzpsi * self.npsi)
+        if 0 < m <= 1:   # phi(k / m) = 0 from k = 2 on: the two-pole recursion
+            self._call("ht_shift_coeffback", self._hc, _lib.ptr(x), _lib.ptr(out), b,
+                       float(np.float32(self.phi(np.float32(1 / m)))))
+            return out
+        fx = np.linspace(-1 / 2, 1 / 2 - 1 / self.npsi, self.npsi).astype("float32")
+        fy = np.linspace(-1 / 2, 1 / 2 - 1 / self.nzpsi, self.nzpsi).astype("float32")
         dx = np.float32(self.phi(0))
         dy = np.float32(self.phi(0))
         for k in range(1, 5):
             pk = np.float32(self.phi(np.float32(k / m)))
-            dx = (dx + 2 * pk * np.cos(2 * np.pi * k * x)).astype("float32")
-            dy = (dy + 2 * pk * np.cos(2 * np.pi * k * y)).astype("float32")
+            dx = (dx + 2 * pk * np.cos(2 * np.pi * k * fx)).astype("float32")
+            dy = (dy + 2 * pk * np.cos(2 * np.pi * k * fy)).astype("float32")
         # FFT order, each axis carrying its 1/N
         symx = torch.from_numpy((1.0 / (self.npsi * np.fft.fftshift(dx).astype(np.float64))).astype("float32"))
         symy = torch.from_numpy((1.0 / (self.nzpsi * np.fft.fftshift(dy).astype(np.float64))).astype("float32"))
         symx, symy = symx.to(psi.device), symy.to(psi.device)
-        x = psi.to(torch.complex64).contiguous()
-        out = torch.empty_like(x)
-        b = x.numel() // (self.nzpsi * self.npsi)
         self._call("ht_shift_filter", self._hc, _lib.ptr(x), _lib.ptr(out), b, _lib.ptr(symx), _lib.ptr(symy))
         return out
 
@@ -171,7 +177,11 @@ class Shift:
             raise ValueError(f"spsi must be [batch, {self.nz}, {self.n}], got {tuple(spsi.shape)}")
         g = spsi.to(torch.complex64).contiguous()
         r = _f32(r, g.device).reshape(-1)
-        m = _f32(m if isinstance(m, (torch.Tensor, np.ndarray)) else np.asarray(m, np.float32), g.device).reshape(-1)
+        if isinstance(m, (float, int)):   # filled on the device: a copy from pageable memory would wait for it
+            m = torch.full((1,), float(m), dtype=torch.float32, device=g.device)
+        else:
+            m = _f32(m if isinstance(m, (torch.Tensor, np.ndarray)) else np.asarray(m, np.float32),
+                     g.device).reshape(-1)
         if m.numel() not in (1, g.shape[0]):
             raise ValueError(f"m must hold 1 or {g.shape[0]} magnifications, got {m.numel()}")
         if r.numel() != 2 * g.shape[0]:

@@ -144,6 +144,13 @@ int ht_shift_destroy(ht_shift_s* s);
 /* out = ifft2(fft2(psi) / B3): the B-spline prefilter (shift.py:74-82);
  * complex64 [batch, nzpsi, npsi]; out may alias psi. */
 int ht_shift_coeff(ht_shift_s* s, const void* psi, void* out, long batch, void* stream);
+/* The prefilter of real images, float32 [batch, nzpsi, npsi] (the real part of
+ * ht_shift_coeff's output for a real psi); out must not overlap psi.  Any handle. */
+int ht_shift_coeff_real(ht_shift_s* s, const float* psi, float* out, long batch, void* stream);
+/* The prefilter of the spline stretched by a magnification m <= 1 (shift.py:84-96):
+ * symbol 1 / ((4 + 2 b cos wy)(4 + 2 b cos wx)) with b = phi(1/m) in [0, 1]; complex64
+ * [batch, nzpsi, npsi]; out must not overlap psi. */
+int ht_shift_coeffback(ht_shift_s* s, const void* psi, void* out, long batch, float b, void* stream);
 /* The z-axis half of the prefilter (the column factor of shift.py:74-82):
  * out = Cz in for in, out [nzpsi, ncols] complex64 (a volume [nzpsi, ny, nx]
  * has ncols = ny nx); out may alias in. */

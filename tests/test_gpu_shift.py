@@ -123,3 +123,90 @@ def test_coeff_large_against_fp64():
     s = Shift(n, n, n, n, "complex64")
     o = O.Shift(n, n, n, n, "complex64", "complex128")
     assert rel_l2(s.coeff(torch.from_numpy(psi).cuda()).cpu().numpy(), o.coeff(psi.astype(np.complex128))) < TOL
+
+
+@pytest.mark.parametrize("dtype", ["complex64", "float32"])
+@pytest.mark.parametrize("npsi,nzpsi", [(18, 24), (36, 64), (96, 128), (192, 48), (384, 256)])
+def test_prefilter_over_tiles(dtype, npsi, nzpsi):
+    """The recursive prefilter at lines shorter than its warm-up, whole tiles and
+    remainders, out of place, in place and along z, against FP64."""
+    from holotomocupy_b200 import Shift, _lib
+    rng = np.random.default_rng(npsi)
+    s = Shift(npsi, npsi, nzpsi, nzpsi, dtype)
+    o = O.Shift(npsi, npsi, nzpsi, nzpsi, dtype, "complex128")
+    psi = rng.standard_normal((3, nzpsi, npsi)).astype("float32")
+    if dtype == "complex64":
+        psi = (psi + 1j * rng.standard_normal(psi.shape)).astype("complex64")
+    got = s.coeff(torch.from_numpy(psi).cuda())
+    assert rel_l2(got.cpu().numpy(), o.coeff(psi.astype(np.complex128))) < 1e-6
+    if dtype == "complex64":
+        x = torch.from_numpy(psi).cuda()
+        _lib.call("ht_shift_coeff", s._hc, _lib.ptr(x), _lib.ptr(x), 3, _lib.stream_ptr())
+        assert rel_l2(x.cpu().numpy(), got.cpu().numpy()) < 1e-6
+        vol = torch.from_numpy(psi[0]).cuda()
+        ref = np.fft.ifft(np.fft.fft(psi[0].astype(np.complex128), axis=0)
+                          / (4 + 2 * np.cos(2 * np.pi * np.arange(nzpsi) / nzpsi))[:, None], axis=0)
+        for out in (torch.empty_like(vol), vol):
+            _lib.call("ht_shift_coeff_z", s._hc, _lib.ptr(vol), _lib.ptr(out), npsi, _lib.stream_ptr())
+            assert rel_l2(out.cpu().numpy(), ref) < 1e-6
+
+
+@pytest.mark.parametrize("mag", [-0.9, 0.3, 0.59, 0.61, 1.0, 1.7, 3.5])
+@pytest.mark.parametrize("dtype", ["complex64", "float32"])
+def test_shift_family_over_tiles_and_magnifications(dtype, mag):
+    """The separable tiles at their edges (odd detectors around 32 x 64 outputs),
+    magnifications that take a tile whole, in parts and pixel by pixel, and an
+    image shifted off the grid, against the FP32 oracle."""
+    from holotomocupy_b200 import Shift
+    rng = np.random.default_rng(int(100 * abs(mag)))
+    n, nz, npsi, nzpsi, nt = 65, 131, 64, 128, 3
+    s = Shift(n, npsi, nz, nzpsi, dtype)
+    o = O.Shift(n, npsi, nz, nzpsi, dtype, "complex64")
+
+    def arr(*shape):
+        a = rng.standard_normal(shape).astype("float32")
+        return a if dtype == "float32" else (a + 1j * rng.standard_normal(shape)).astype("complex64")
+    c, c1, c2 = (arr(nt, nzpsi, npsi) for _ in range(3))
+    g = arr(nt, nz, n)
+    r, d1, d2 = (rng.uniform(-4, 4, (nt, 2)).astype("float32") for _ in range(3))
+    r[2] = (1e4, -1e4)
+    m = np.full(nt, mag, "float32")
+    cu = lambda a: torch.from_numpy(a).cuda()
+    dp, dr = s.dcurlySadjc(cu(c), cu(r), cu(m), cu(g))
+    rp, rr = o.dcurlySadjc(c, r, m, g)
+    for got, ref in ((s.S(cu(c), cu(r), cu(m)), o.S(c, r, m)),
+                     (s.dcurlySc(cu(c), cu(r), cu(m), cu(c1), cu(d1)), o.dcurlySc(c, r, m, c1, d1)),
+                     (s.d2curlySc(cu(c), cu(r), cu(m), cu(c1), cu(d1), cu(c2), cu(d2)),
+                      o.d2curlySc(c, r, m, c1, d1, c2, d2)),
+                     (s.Sadj(cu(g), cu(r), cu(m)), o.Sadj(g, r, m)), (dp, rp), (dr, rr)):
+        assert rel_l2(got.cpu().numpy(), ref) < TOL, rel_l2(got.cpu().numpy(), ref)
+        assert not got[2].any()
+
+
+@pytest.mark.parametrize("m", [0.26, 0.4, 0.74, 0.8, 1.3])
+def test_sback_over_tiles(m):
+    """Sback across the edges of its 32 x 64 tiles, whole and in parts."""
+    from holotomocupy_b200 import Shift
+    rng = np.random.default_rng(5)
+    n, npsi, nz, nzpsi, nt = 70, 96, 150, 192, 2
+    g = (rng.standard_normal((nt, nz, n)) + 1j * rng.standard_normal((nt, nz, n))).astype("complex64")
+    r = rng.uniform(-3, 3, (nt, 2)).astype("float32")
+    s = Shift(n, npsi, nz, nzpsi, "complex64")
+    o = O.Shift(n, npsi, nz, nzpsi, "complex64", "complex64")
+    got = s.Sback(torch.from_numpy(g).cuda(), torch.from_numpy(r).cuda(), m).cpu().numpy()
+    # a tap range at its rounding boundary may differ by one tap between two FP32 evaluations of the position
+    assert rel_l2(got, o.Sback(g, r, np.float32(m))) < (5e-5 if m < 0.5 else TOL)
+
+
+@pytest.mark.parametrize("m", [0.3, 0.5, 0.51, 0.75, 0.999, 1.0])
+def test_coeffback_recursion_matches_its_symbol(m):
+    """The two-pole form of the stretched prefilter (m <= 1) against its symbol in FP64."""
+    from holotomocupy_b200 import Shift
+    rng = np.random.default_rng(3)
+    npsi, nzpsi = 96, 64
+    psi = (rng.standard_normal((2, nzpsi, npsi)) + 1j * rng.standard_normal((2, nzpsi, npsi))).astype("complex64")
+    s = Shift(npsi, npsi, nzpsi, nzpsi, "complex64")
+    sym = [4 + sum(2 * s.phi(k / m) * np.cos(2 * np.pi * k * np.arange(n) / n) for k in range(1, 5))
+           for n in (nzpsi, npsi)]
+    ref = np.fft.ifft2(np.fft.fft2(psi.astype(np.complex128)) / np.outer(*sym))
+    assert rel_l2(s.coeffback(torch.from_numpy(psi).cuda(), m).cpu().numpy(), ref) < 1e-6
