@@ -38,6 +38,8 @@ SIGNATURES = {
     "ht_tomo_RT_coeffx": [_vp, _vp, _vp, _c_int, _c_float, _vp],
     "ht_tomo_R_slab": [_vp, _vp, _vp, _c_int, _c_int, _c_int, _vp],
     "ht_tomo_RT_slab": [_vp, _vp, _vp, _c_int, _c_int, _c_int, _c_float, _vp],
+    "ht_tomo_R_real": [_vp, _vp, _vp, _c_int, _c_int, _vp],
+    "ht_tomo_RT_filter": [_vp, _vp, _vp, _c_int, _c_int, _c_int, _vp, _c_float, _vp],
     "ht_shift_create": [_c_int, _c_int, _c_int, _c_int, _c_int, ctypes.POINTER(_vp)],
     "ht_shift_destroy": [_vp],
     "ht_shift_coeff": [_vp, _vp, _vp, _c_long, _vp],

@@ -234,6 +234,25 @@ struct SplitView {
   __device__ __forceinline__ void st(int k, float2 v) const { s.st(k, v); }
 };
 
+// A view of a zero-padded line declares kCentralHalf: only its samples N/4 <= k <
+// 3N/4 are data (loads) or wanted (stores), and its ld / st are called for those
+// alone where a radix that is a multiple of 4 makes that known at compile time
+// (sample b + j N/R lies in the j-th of R parts).
+template <class V, class = void>
+struct central_half : std::false_type {};
+template <class V>
+struct central_half<V, std::void_t<decltype(V::kCentralHalf)>> : std::true_type {};
+template <class L, class S>
+struct central_half<SplitView<L, S>, void> : std::false_type {};
+template <class V>
+struct load_half : central_half<V> {};
+template <class L, class S>
+struct load_half<SplitView<L, S>> : central_half<L> {};
+template <class V>
+struct store_half : central_half<V> {};
+template <class L, class S>
+struct store_half<SplitView<L, S>> : central_half<S> {};
+
 // ------------------------------------------------------------- one stage
 // tw4: table of exp(-2 pi i m / (4N)); W_N^a = tw4[4a].  SYNC_MID: barrier
 // between the loads and the stores (needed when both are the same shared
@@ -256,7 +275,12 @@ __device__ __forceinline__ void fft_stage(float2 (&v)[E], const SM& sm, int t,
       for (int j = 0; j < R; ++j) v[s * R + j] = sm.ld_pad(pb + j * (NR + NR / 16));
     } else {
 #pragma unroll
-      for (int j = 0; j < R; ++j) v[s * R + j] = sm.ld(b + j * NR);
+      for (int j = 0; j < R; ++j) {
+        if (load_half<SM>::value && R % 4 == 0 && (j < R / 4 || j >= 3 * R / 4))
+          v[s * R + j] = make_float2(0.f, 0.f);
+        else
+          v[s * R + j] = sm.ld(b + j * NR);
+      }
     }
   }
 #pragma unroll
@@ -283,7 +307,10 @@ __device__ __forceinline__ void fft_stage(float2 (&v)[E], const SM& sm, int t,
       for (int j = 0; j < R; ++j) sm.st_pad(pk + j * (P + P / 16), v[s * R + j]);
     } else {
 #pragma unroll
-      for (int j = 0; j < R; ++j) sm.st((b - i) * R + i + j * P, v[s * R + j]);
+      for (int j = 0; j < R; ++j) {
+        if (store_half<SM>::value && P * R == N && R % 4 == 0 && (j < R / 4 || j >= 3 * R / 4)) continue;
+        sm.st((b - i) * R + i + j * P, v[s * R + j]);
+      }
     }
   }
   if constexpr (SYNC_END) sync();

@@ -94,25 +94,44 @@ class Tomo:
             yield z0, min(self._nz, nz - z0)
 
     def _R_into(self, x, res, coeffx=False):
-        """res[ntheta, nz, n] = R(x[nz, n, n]) (complex64, contiguous), with the
-        detector-axis B-spline prefilter when coeffx (ht_tomo_R_slab)."""
+        """res[ntheta, nz, n] = R(x[nz, n, n]) (both complex64 or both float32,
+        contiguous), with the detector-axis B-spline prefilter when coeffx
+        (complex64 only; ht_tomo_R_slab)."""
         nz, st = x.shape[0], _lib.stream_ptr()
-        row = self.n * 8
+        row = self.n * x.element_size()
         with torch.cuda.device(x.device):
             for z0, nzs in self._slabs(nz):
-                _lib.call("ht_tomo_R_slab", self._h, _lib.ptr(x[z0]), ctypes.c_void_p(res.data_ptr() + z0 * row), nzs,
-                          nz, int(coeffx), st)
+                src, dst = _lib.ptr(x[z0]), ctypes.c_void_p(res.data_ptr() + z0 * row)
+                if x.is_complex():
+                    _lib.call("ht_tomo_R_slab", self._h, src, dst, nzs, nz, int(coeffx), st)
+                else:
+                    _lib.call("ht_tomo_R_real", self._h, src, dst, nzs, nz, st)
         return res
 
-    def _RT_into(self, d, res, coeffx=False, scale=1.0):
-        """res[nz, n, n] = scale R^T(d[ntheta, nz, n]) (complex64, contiguous)."""
+    def _RT_into(self, d, res, coeffx=False, scale=1.0, sym=None):
+        """res[nz, n, n] = scale R^T(d[ntheta, nz, n]) (both complex64 or both
+        float32, contiguous), after the detector-axis B-spline prefilter
+        (coeffx, complex64 only) or the filter of symbol sym."""
         nz, st = d.shape[1], _lib.stream_ptr()
-        row = self.n * 8
+        row = self.n * d.element_size()
         with torch.cuda.device(d.device):
             for z0, nzs in self._slabs(nz):
-                _lib.call("ht_tomo_RT_slab", self._h, ctypes.c_void_p(d.data_ptr() + z0 * row), _lib.ptr(res[z0]),
-                          nzs, nz, int(coeffx), float(scale), st)
+                src, dst = ctypes.c_void_p(d.data_ptr() + z0 * row), _lib.ptr(res[z0])
+                if coeffx:
+                    _lib.call("ht_tomo_RT_slab", self._h, src, dst, nzs, nz, 1, float(scale), st)
+                else:
+                    _lib.call("ht_tomo_RT_filter", self._h, src, dst, nzs, nz, int(not d.is_complex()),
+                              _lib.ptr(sym) if sym is not None else None, float(scale), st)
         return res
+
+    @staticmethod
+    def _result(out, shape, dtype, device):
+        """(the array an operator writes, whether out still has to be copied from it)"""
+        if out is None:
+            return torch.empty(shape, dtype=dtype, device=device), False
+        if dtype.is_complex or (out.dtype == dtype and out.is_contiguous() and tuple(out.shape) == tuple(shape)):
+            return out, False
+        return torch.empty(shape, dtype=dtype, device=device), True
 
     def R(self, obj, out=None):
         """Radon transform (tomo.py:56-86): [nz, n, n] -> [ntheta, nz, n] (any nz:
@@ -121,38 +140,28 @@ class Tomo:
         nz = obj.shape[0]
         if tuple(obj.shape[1:]) != (self.n, self.n):
             raise ValueError(f"obj must be [nz, {self.n}, {self.n}], got {tuple(obj.shape)}")
-        real = not obj.is_complex()
-        x = obj.to(torch.complex64).contiguous()
-        res = out if (out is not None and not real) else torch.empty(self.ntheta, nz, self.n, dtype=torch.complex64,
-                                                                     device=x.device)
+        x = obj.to(torch.complex64 if obj.is_complex() else torch.float32).contiguous()
+        res, copy = self._result(out, (self.ntheta, nz, self.n), x.dtype, x.device)
         self._R_into(x, res)
-        if real:
-            res = res.real.contiguous()
-            if out is not None:
-                out.copy_(res)
-                return out
-        return res
+        return out.copy_(res) if copy else res
 
     def RT(self, data, out=None):
         """Adjoint Radon transform (tomo.py:88-116): [ntheta, nz, n] -> [nz, n, n]."""
+        return self._back(data, out)
+
+    def _back(self, data, out=None, scale=1.0, sym=None):
         _lib.require_cuda(data, "data")
         nz = data.shape[1]
         if data.shape[0] != self.ntheta or data.shape[2] != self.n:
             raise ValueError(f"data must be [{self.ntheta}, nz, {self.n}], got {tuple(data.shape)}")
-        real = not data.is_complex()
-        x = data.to(torch.complex64).contiguous()
-        res = out if (out is not None and not real) else torch.empty(nz, self.n, self.n, dtype=torch.complex64,
-                                                                     device=x.device)
-        self._RT_into(x, res)
-        if real:
-            res = res.real.contiguous()
-            if out is not None:
-                out.copy_(res)
-                return out
-        return res
+        x = data.to(torch.complex64 if data.is_complex() else torch.float32).contiguous()
+        res, copy = self._result(out, (nz, self.n, self.n), x.dtype, x.device)
+        self._RT_into(x, res, scale=scale, sym=sym)
+        return out.copy_(res) if copy else res
 
-    def _filter_sino(self, data, filter_name):
-        """1-D detector filter of tomo.py:118-161 (ramp, shepp, parzen)."""
+    def _filter_symbol(self, filter_name):
+        """The detector filter's symbol / n (tomo.py:118-161: ramp, shepp,
+        parzen) in FFT order, on the device."""
         n = self.n
         if filter_name not in self._filters:
             f = np.fft.fftfreq(n).astype("float32")
@@ -167,7 +176,12 @@ class Tomo:
             else:
                 raise ValueError(f"Unknown filter '{filter_name}'. Choose: ramp, shepp, parzen.")
             self._filters[filter_name] = torch.from_numpy((h / n).astype("float32")).to(self.device)
-        sym = self._filters[filter_name]
+        return self._filters[filter_name]
+
+    def _filter_sino(self, data, filter_name):
+        """1-D detector filter of tomo.py:118-161 (ramp, shepp, parzen)."""
+        n = self.n
+        sym = self._filter_symbol(filter_name)
         real = not data.is_complex()
         x = data.to(torch.complex64).contiguous()
         out = torch.empty_like(x)
@@ -181,9 +195,8 @@ class Tomo:
         if isinstance(data, np.ndarray):
             data = torch.from_numpy(data).to(self.device)
         norm_const = float(np.float32(np.sqrt(self.n / self.ntheta)))
-        res = self.RT(self._filter_sino(data, filter_name))
-        res *= norm_const
-        return res
+        # the filter is diagonal in the spectrum R^T starts from; its symbol carries the 1/n of an inverse FFT
+        return self._back(data, scale=self.n * norm_const, sym=self._filter_symbol(filter_name))
 
     def rec_tomo(self, d, niter=1):
         """Conjugate-gradient tomography (tomo.py:185-210), FP64 inner products."""

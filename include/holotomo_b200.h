@@ -107,6 +107,15 @@ int ht_tomo_R(ht_tomo_s* t, const void* obj, void* sino, int nz, void* stream);
 
 /* obj[nz, n, n] = R^T(sino[ntheta, nz, n]), complex64 (tomo.py:88-116). */
 int ht_tomo_RT(ht_tomo_s* t, const void* sino, void* obj, int nz, void* stream);
+/* R of real volumes: float32 obj [nz, n, n] to sino [ntheta, nz, n], the real part of
+ * ht_tomo_R's output; ldz >= nz rows an angle in sino. */
+int ht_tomo_R_real(ht_tomo_s* t, const float* obj, float* sino, int nz, int ldz, void* stream);
+/* obj = scale * R^T(F sino), F the circulant filter along the detector axis with the
+ * real even symbol sym [n] in FFT order on the device (NULL: none), applied in R^T's
+ * own detector spectrum: filtered back-projection (tomo.py:118-183) without a pass
+ * for the filter.  is_real: float32 arrays (the real part), else complex64. */
+int ht_tomo_RT_filter(ht_tomo_s* t, const void* sino, void* obj, int nz, int ldz, int is_real, const float* sym,
+                      float scale, void* stream);
 /* R followed by the detector-axis half of the B-spline prefilter, and R^T
  * preceded by it: Cx(R obj) and R^T(Cx sino), Cx the circulant filter with
  * symbol 1 / (4 + 2 cos 2 pi k / n) along the last axis (shift.py:74-82, its

@@ -158,3 +158,23 @@ def test_R_RT_by_slabs_equal_whole_volume():
     whole, slabs = Tomo(n, nz, theta, 0.9), Tomo(n, 8, theta, 0.9)
     assert rel_l2(slabs.R(x).cpu().numpy(), whole.R(x).cpu().numpy()) < 1e-7
     assert rel_l2(slabs.RT(y).cpu().numpy(), whole.RT(y).cpu().numpy()) < 1e-7
+
+
+@pytest.mark.parametrize("n,ntheta,nz", [(18, 20, 1), (24, 5, 4), (32, 100, 5), (48, 33, 8), (64, 150, 9),
+                                         (64, 7, 16), (96, 31, 17), (128, 400, 33)])
+def test_R_RT_over_slice_batches(n, ntheta, nz):
+    """Slice counts around the interleaves of 4, 8 and 16, and angles from dense
+    (neighbouring lines share windows; lists near the centre longer than a
+    lane group takes) to sparse and unsorted, against the oracle."""
+    from holotomocupy_b200 import Tomo
+    rng = np.random.default_rng(n + nz)
+    theta = np.linspace(0, np.pi, ntheta, endpoint=False)
+    if nz % 2:
+        theta = rng.permutation(theta + rng.uniform(-0.4, 0.4, ntheta) * np.pi / ntheta) + 2 * np.pi * (nz % 3 - 1)
+    theta = theta.astype("float32")
+    t = Tomo(n, nz, theta, 1)
+    o = O.Tomo(n, nz, theta, 1, "complex64")
+    x = (rng.standard_normal((nz, n, n)) + 1j * rng.standard_normal((nz, n, n))).astype("complex64")
+    y = (rng.standard_normal((ntheta, nz, n)) + 1j * rng.standard_normal((ntheta, nz, n))).astype("complex64")
+    assert rel_l2(t.R(torch.from_numpy(x).cuda()).cpu().numpy(), o.R(x)) < TOL
+    assert rel_l2(t.RT(torch.from_numpy(y).cuda()).cpu().numpy(), o.RT(y)) < TOL
