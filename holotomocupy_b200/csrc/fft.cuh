@@ -82,6 +82,41 @@ struct Dft<8, INV> {
   }
 };
 
+// 16 points as 4 x 4: two rounds of radix-4 with the W16 twiddles between.
+template <bool INV>
+struct Dft<16, INV> {
+  static __device__ __forceinline__ float2 tw(float2 a, float c, float s) {  // a * (c - i s), conjugated for INV
+    return INV ? make_float2(a.x * c - a.y * s, a.y * c + a.x * s) : make_float2(a.x * c + a.y * s, a.y * c - a.x * s);
+  }
+  static __device__ __forceinline__ void run(float2* v) {
+    const float c1 = 0.92387953251128675613f, s1 = 0.38268343236508977173f, r = 0.70710678118654752440f;
+    float2 a[4][4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {  // columns q: v[q + 4 p]
+#pragma unroll
+      for (int p = 0; p < 4; ++p) a[q][p] = v[q + 4 * p];
+      Dft<4, INV>::run(a[q]);
+    }
+    // times W16^(q k)
+    a[1][1] = tw(a[1][1], c1, s1);
+    a[1][2] = tw(a[1][2], r, r);
+    a[1][3] = tw(a[1][3], s1, c1);
+    a[2][1] = tw(a[2][1], r, r);
+    a[2][2] = rot<INV>(a[2][2]);
+    a[2][3] = tw(a[2][3], -r, r);
+    a[3][1] = tw(a[3][1], s1, c1);
+    a[3][2] = tw(a[3][2], -r, r);
+    a[3][3] = tw(a[3][3], -c1, -s1);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      float2 b[4] = {a[0][k], a[1][k], a[2][k], a[3][k]};
+      Dft<4, INV>::run(b);
+#pragma unroll
+      for (int p = 0; p < 4; ++p) v[k + 4 * p] = b[p];
+    }
+  }
+};
+
 // ----------------------------------------------------- shared-memory views
 // Row line: contiguous, one pad slot every 16 samples (bank-conflict free for
 // the stride-R writes of the first stages).
@@ -142,11 +177,11 @@ HT_PLAN(256, 8, 8, 8, 4)
 HT_PLAN(384, 12, 4, 4, 4, 3, 2)   // 12 samples a thread: the stencil row kernels keep their occupancy
 HT_PLAN(512, 8, 8, 8, 8)
 HT_PLAN(768, 12, 4, 4, 4, 4, 3)
-HT_PLAN(1024, 16, 8, 8, 8, 2)
+HT_PLAN(1024, 16, 16, 16, 4)
 HT_PLAN(1536, 24, 8, 8, 8, 3)
-HT_PLAN(2048, 16, 8, 8, 8, 4)
+HT_PLAN(2048, 16, 16, 16, 8)
 HT_PLAN(3072, 24, 8, 8, 8, 2, 3)
-HT_PLAN(4096, 16, 8, 8, 8, 8)
+HT_PLAN(4096, 16, 16, 16, 16)
 #undef HT_PLAN
 
 // ColPlan<N>: the plan of the column passes (a tile of columns per CTA, no
@@ -223,6 +258,19 @@ __device__ __forceinline__ void twiddles(const float2* __restrict__ tw4, int a, 
     }
   }
 }
+// Radix 16: W^a, W^2a, W^4a and W^8a are read, so that every other power is a
+// product of at most four of them.
+template <int N, bool INV>
+__device__ __forceinline__ void twiddles16(const float2* __restrict__ tw4, int a, float2 (&w)[16]) {
+  w[0] = make_float2(1.f, 0.f);
+#pragma unroll
+  for (int k = 1; k < 16; k *= 2) {
+    w[k] = __ldg(&tw4[4 * ((k * a) % N)]);
+    if (INV) w[k].y = -w[k].y;
+#pragma unroll
+    for (int j = 1; j < k; ++j) w[k + j] = cmul(w[j], w[k]);
+  }
+}
 
 // Loads through one view, stores through another: a first stage that reads
 // its line from global memory, or a last stage that writes it there.
@@ -265,7 +313,7 @@ __device__ __forceinline__ void fft_stage(float2 (&v)[E], const SM& sm, int t,
   constexpr int NB = E / R;
   constexpr int NR = N / R;
   static_assert(E % R == 0, "radix must divide the samples per thread");
-  static_assert(R <= 8, "twiddles() covers radices up to 8");
+  static_assert(R <= 8 || R == 16, "twiddles() covers radices up to 8, and 16");
 #pragma unroll
   for (int s = 0; s < NB; ++s) {
     const int b = t + s * T;
@@ -289,7 +337,10 @@ __device__ __forceinline__ void fft_stage(float2 (&v)[E], const SM& sm, int t,
     if constexpr (P > 1) {
       const int i = b % P;
       float2 w[R];
-      twiddles<R, INV>(tw4, i * (N / (P * R)), N, w);
+      if constexpr (R == 16)
+        twiddles16<N, INV>(tw4, i * (N / (P * R)), w);
+      else
+        twiddles<R, INV>(tw4, i * (N / (P * R)), N, w);
 #pragma unroll
       for (int j = 1; j < R; ++j) v[s * R + j] = cmul(v[s * R + j], w[j]);
     }

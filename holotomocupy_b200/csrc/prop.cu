@@ -30,7 +30,24 @@
 namespace ht {
 
 // ------------------------------------------------------------ row DCT-II
-// in, out: [nrows, N]; out may alias in.
+// A row of an image at position k of the reordered sequence.
+template <int N>
+struct RowIn {
+  const float2* p;
+  __device__ __forceinline__ float2 ld(int k) const { return p[dct_sample_at(k, N)]; }
+};
+template <int N>
+struct RowOut {
+  float2* p;
+  bool valid;
+  __device__ __forceinline__ void st(int k, float2 v) const {
+    if (valid) p[dct_sample_at(k, N)] = v;
+  }
+};
+
+// in, out: [nrows, N]; out may alias in (a line's loads come before its first
+// store).  The first FFT stage loads from global memory, the output combine
+// stores there: a sample passes shared memory between the stages only.
 template <int N>
 __global__ void __launch_bounds__(RowCfg<N>::THREADS)
 k_dct2_rows(const float2* in, float2* out, long nrows, const float2* __restrict__ tw4) {
@@ -41,13 +58,13 @@ k_dct2_rows(const float2* in, float2* out, long nrows, const float2* __restrict_
   const long row = (long)blockIdx.x * RowCfg<N>::LINES + line;
   const bool valid = row < nrows;
   SmRow sm{smem + line * LS};
-  const float2* src = in + row * N;
-  for (int g = t; g < N; g += T) sm.st(dct_perm_inv(g, N), valid ? src[g] : make_float2(0.f, 0.f));
-  __syncthreads();
-  fft_line<N, false>(sm, t, tw4, line_sync<T>());
+  fft_line_from<N, false>(RowIn<N>{in + (valid ? row : nrows - 1) * N}, sm, t, tw4, line_sync<T>());
   if (!valid) return;
   float2* dst = out + row * N;
-  for (int k = t; k <= N / 2; k += T) {
+#pragma unroll
+  for (int i = 0; i <= (N / 2) / T; ++i) {
+    const int k = t + i * T;
+    if (k > N / 2) break;
     const float2 A = sm.ld(k), B = sm.ld(k == 0 ? 0 : N - k);
     const float2 w = __ldg(&tw4[k]);
     const float2 P = cmul(w, A), Q = cmulc(B, w);
@@ -57,6 +74,8 @@ k_dct2_rows(const float2* in, float2* out, long nrows, const float2* __restrict_
 }
 
 // ----------------------------------------------------------- row DCT-III
+// The combine loads a line's samples in pairs, all before its first store; the
+// last FFT stage stores to global memory.
 template <int N>
 __global__ void __launch_bounds__(RowCfg<N>::THREADS)
 k_dct3_rows(const float2* in, float2* out, long nrows, const float2* __restrict__ tw4) {
@@ -67,25 +86,61 @@ k_dct3_rows(const float2* in, float2* out, long nrows, const float2* __restrict_
   const long row = (long)blockIdx.x * RowCfg<N>::LINES + line;
   const bool valid = row < nrows;
   SmRow sm{smem + line * LS};
-  const float2* src = in + row * N;
-  for (int m = t; m <= N / 2; m += T) {
-    const float2 z = make_float2(0.f, 0.f);
-    const float2 G = valid ? src[m] : z;
-    const float2 H = valid ? src[m == 0 ? 0 : N - m] : z;
+  const float2* src = in + (valid ? row : nrows - 1) * N;
+  constexpr int NM = (N / 2) / T + 1;  // m = t + i T covers 0..N/2
+  float2 G[NM], H[NM];
+#pragma unroll
+  for (int i = 0; i < NM; ++i) {
+    const int m = min(t + i * T, N / 2);
+    G[i] = src[m];
+    H[i] = src[m == 0 ? 0 : N - m];
+  }
+#pragma unroll
+  for (int i = 0; i < NM; ++i) {
+    const int m = t + i * T;
+    if (m > N / 2) break;
     if (m == 0) {
-      sm.st(0, G);
+      sm.st(0, G[i]);
     } else {
       const float2 w = __ldg(&tw4[m]);
       // V'[m] = 1/2 w^m (G[m] + i G[N-m]);  V'[N-m] = 1/2 conj(w^m) (G[m] - i G[N-m])
-      sm.st(m, cscale(cmul(w, cadd(G, cmul_i(H))), 0.5f));
-      if (m != N / 2) sm.st(N - m, cscale(cmulc(csub(G, cmul_i(H)), w), 0.5f));
+      sm.st(m, cscale(cmul(w, cadd(G[i], cmul_i(H[i]))), 0.5f));
+      if (m != N / 2) sm.st(N - m, cscale(cmulc(csub(G[i], cmul_i(H[i])), w), 0.5f));
     }
   }
-  __syncthreads();
-  fft_line<N, false>(sm, t, tw4, line_sync<T>());
-  if (!valid) return;
-  float2* dst = out + row * N;
-  for (int g = t; g < N; g += T) dst[g] = sm.ld(dct_perm(g, N));
+  line_sync<T>()();
+  fft_line_to<N, false>(sm, RowOut<N>{out + row * N, valid}, t, tw4, line_sync<T>());
+}
+
+// Rows of 512 samples, a warp a row, on the register transforms of row512.cuh:
+// the combines happen in registers too.
+constexpr int kP512Lines = 4;
+__global__ void __launch_bounds__(32 * kP512Lines)
+k_dct2_rows512(const float2* in, float2* out, long nrows, const float2* __restrict__ tw4) {
+  __shared__ float2 smem[kP512Lines * SmRow::padded(kR512)];
+  const int line = threadIdx.x / 32, t = threadIdx.x % 32;
+  const long row = (long)blockIdx.x * kP512Lines + line;
+  if (row >= nrows) return;
+  SmRow sm{smem + line * SmRow::padded(kR512)};
+  const float2* src = in + row * kR512;
+  float2 v[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = src[dct_sample_at(r512_pos(t, i), kR512)];
+  r512_dct2_tail(v, sm, t, tw4, out + row * kR512, true);
+}
+__global__ void __launch_bounds__(32 * kP512Lines)
+k_dct3_rows512(const float2* in, float2* out, long nrows, const float2* __restrict__ tw4) {
+  __shared__ float2 smem[kP512Lines * SmRow::padded(kR512)];
+  const int line = threadIdx.x / 32, t = threadIdx.x % 32;
+  const long row = (long)blockIdx.x * kP512Lines + line;
+  if (row >= nrows) return;
+  SmRow sm{smem + line * SmRow::padded(kR512)};
+  float2 v[16];
+  r512_dct3_head(v, in + row * kR512, true, sm, t, tw4);
+  r512_finish_to_regs(v, sm, t, tw4);
+  float2* dst = out + row * kR512;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) dst[dct_sample_at(r512_pos(t, i), kR512)] = v[i];
 }
 
 // ------------------------------------- column DCT-II, x table, DCT-III
@@ -265,6 +320,12 @@ k_dct_cols512(float2* data, int n, const float2* __restrict__ Hall, int ntab, co
 template <int N>
 static cudaError_t launch_dct_rows(bool inverse, const float2* in, float2* out, long nrows,
                                    const float2* tw4, cudaStream_t st) {
+  if constexpr (N == kR512) {
+    const auto kern = inverse ? k_dct3_rows512 : k_dct2_rows512;
+    kern<<<(unsigned)((nrows + kP512Lines - 1) / kP512Lines), 32 * kP512Lines, 0, st>>>(in, out, nrows, tw4);
+    ::ht::count_launch();
+    return cudaGetLastError();
+  }
   using CF = RowCfg<N>;
   const long grid = (nrows + CF::LINES - 1) / CF::LINES;
   if (inverse) {

@@ -91,3 +91,22 @@ def test_in_place_and_aliasing():
     y = x.clone()
     _lib.call("ht_prop_D", p._h, _lib.ptr(y), _lib.ptr(y), 3, 0, _lib.stream_ptr())
     torch.testing.assert_close(y, ref, rtol=0, atol=0)
+
+
+@pytest.mark.parametrize("n,nz,batch", [(18, 24, 1), (96, 512, 3), (512, 36, 7), (1024, 64, 2), (64, 2048, 3),
+                                        (4096, 18, 1)])
+def test_row_passes_in_place_and_out_of_place(n, nz, batch):
+    """The row passes at each kind of line (several lines a block and a ragged
+    last block, a warp a line, a block a line), in place and out of place: the
+    same samples, and D against the FP64 oracle."""
+    from holotomocupy_b200 import Propagation, _lib
+    rng = np.random.default_rng(n + nz)
+    x = (rng.standard_normal((batch, nz, n)) + 1j * rng.standard_normal((batch, nz, n))).astype("complex64")
+    dist = np.array([3e-3, 6e-3])
+    p = Propagation(n, nz, batch, 2, 7.3e-11, 20e-9, dist)
+    o = O.Propagation(n, nz, batch, 2, 7.3e-11, 20e-9, dist, dtype="complex128")
+    xt = torch.from_numpy(x).cuda()
+    y = xt.clone()
+    _lib.call("ht_prop_D", p._h, _lib.ptr(y), _lib.ptr(y), batch, 1, _lib.stream_ptr())
+    assert torch.equal(y, p.D(xt, 1))
+    assert rel_l2(y.cpu().numpy(), o.D(x.astype(np.complex128), 1)) < TOL_FP64
