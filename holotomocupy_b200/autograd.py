@@ -21,10 +21,15 @@ over (angle, distance) images, optionally in angle chunks whose forward is
 recomputed in the backward pass (``torch.utils.checkpoint``), so that only one
 chunk's intermediates are held at a time.
 """
+import contextlib
+import ctypes
+import threading
+
 import numpy as np
 import torch
 from torch.utils.checkpoint import checkpoint
 
+from . import _lib
 from .propagation import Propagation
 from .shift import Shift
 from .tomo import Tomo
@@ -89,6 +94,75 @@ class _ProbeMul(torch.autograd.Function):
         return gprb, gx
 
 
+class _ChunkMisfit(torch.autograd.Function):
+    """1/N sum (|D_k(prb_k exp(i S_k(coeff(x))))| - d)^2 of one angle chunk by the
+    fused cascade (ht_rec_forward; ht_rec_gradient in the backward pass, which
+    repeats the forward from the saved inputs, so that no image stack is held
+    between the two).  x is the chunk's projections, or with tomo the object."""
+
+    @staticmethod
+    def forward(ctx, x, prb, pos, mag, data, term, tomo):
+        ctx.term, ctx.tomo = term, tomo
+        ctx.save_for_backward(x, prb, pos, mag, data)
+        c = term.sh.coeff(x if tomo is None else tomo.R(x.contiguous()))
+        f = torch.empty(1, dtype=torch.float64, device=x.device)
+        with term.handle(len(pos)) as h:
+            _lib.call("ht_rec_forward", h, _lib.ptr(c), _lib.ptr(pos), _lib.ptr(mag), _lib.ptr(prb), _lib.ptr(data),
+                      None, _lib.ptr(f), _lib.stream_ptr())
+        return (f[0] / term.data_size).to(torch.float32)
+
+    @staticmethod
+    def backward(ctx, g):
+        x, prb, pos, mag, data = ctx.saved_tensors
+        term, tomo = ctx.term, ctx.tomo
+        c = term.sh.coeff(x if tomo is None else tomo.R(x.contiguous()))
+        gc, gpos, gprb = torch.empty_like(c), torch.empty_like(pos), torch.empty_like(prb)
+        with term.handle(len(pos)) as h:
+            _lib.call("ht_rec_gradient", h, _lib.ptr(c), _lib.ptr(pos), _lib.ptr(mag), _lib.ptr(prb),
+                      _lib.ptr(data), _lib.ptr(gc), _lib.ptr(gpos), _lib.ptr(gprb), None, 1.0, 1.0, 0,
+                      _lib.stream_ptr())
+        gx = None
+        if ctx.needs_input_grad[0]:
+            gx = term.sh.coeff(gc)
+            gx = (gx if tomo is None else tomo.RT(gx)) * g
+        return (gx, gprb * g if ctx.needs_input_grad[1] else None, gpos * g if ctx.needs_input_grad[2] else None,
+                None, None, None, None)
+
+
+class _Handles:
+    """Fused-cascade handles of one DataFidelity, by (angles, stream): a handle's
+    workspace serves one call at a time, and calls on one stream run in order.
+    The four last used are kept."""
+
+    KEEP = 4
+
+    def __init__(self):
+        self.lock = threading.Lock()
+        self.items = {}
+
+    def take(self, key, make):
+        with self.lock:
+            h = self.items.pop(key, None)
+        return h if h is not None else make()
+
+    def put(self, key, h):
+        with self.lock:
+            old = self.items.pop(key, None)
+            self.items[key] = h
+            extra = [] if old is None else [old]
+            while len(self.items) > self.KEEP:
+                extra.append(self.items.pop(next(iter(self.items))))
+        for e in extra:
+            _lib.lib().ht_rec_destroy(e)
+
+    def __del__(self):
+        for h in self.items.values():
+            try:
+                _lib.lib().ht_rec_destroy(h)
+            except Exception:
+                pass
+
+
 def radon(obj, tomo):
     """R obj for obj [nz, n, n] complex64 -> [ntheta, nz, n]."""
     return _Radon.apply(obj, tomo)
@@ -113,6 +187,8 @@ class DataFidelity(torch.nn.Module):
     ``chunk`` the angles are processed ``chunk`` at a time and each chunk's
     forward is recomputed during the backward pass."""
 
+    FUSED_ROWS = (32, 64, 128, 256, 384, 512, 768, 1024, 2048)   # detector row lengths of the fused cascade
+
     def __init__(self, sh, prop, theta, mask_r, nobj, nzobj, chunk=None):
         super().__init__()
         theta = np.asarray(theta.cpu() if isinstance(theta, torch.Tensor) else theta, dtype="float32")
@@ -124,6 +200,7 @@ class DataFidelity(torch.nn.Module):
         self.bounds = [(a, min(a + self.chunk, self.ntheta)) for a in range(0, self.ntheta, self.chunk)]
         self.tomos = [Tomo(nobj, nzobj, theta[a:b], mask_r, norm_ntheta=self.ntheta) for a, b in self.bounds]
         self.sh, self.prop = sh, prop
+        self._handles = _Handles()
 
     @classmethod
     def create(cls, n, nz, nobj, nzobj, theta, ndist, wavelength, voxelsize, distance, mask_r=None, chunk=None,
@@ -139,6 +216,43 @@ class DataFidelity(torch.nn.Module):
         """The data term of a Rec (its shift and propagation operators, angles
         and object mask)."""
         return cls(rec.cl_shift, rec.cl_prop, rec.cl_tomo.theta, rec.mask, rec.nobj, rec.nzobj, chunk)
+
+    # ------------------------------------------------ the fused cascade
+    def _use_fused(self, x, prb, pos, mag, data, proj):
+        """The fused cascade takes detectors of its row lengths under objects of
+        up to twice their width (its rows' shared memory), contiguous arrays
+        of the operators' types on their device, and gives no gradient for the
+        data or the magnifications; a handle is not made while a graph is being
+        captured.  Anything else goes operator by operator."""
+        odt = torch.complex64 if self.sh.obj_dtype == "complex64" else torch.float32
+        shape = (self.ntheta, self.nzobj, self.nobj) if proj else (self.nzobj, self.nobj, self.nobj)
+        nd, f32 = (self.ndist, self.nz, self.n), torch.float32
+        want = ((x, odt, shape), (prb, torch.complex64, nd), (pos, f32, (self.ntheta, self.ndist, 2)),
+                (mag, f32, (self.ntheta, self.ndist)), (data, f32, (self.ntheta,) + nd))
+        return (self.n in self.FUSED_ROWS and self.nobj <= 2 * self.n and not data.requires_grad
+                and all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.dtype == dt and tuple(t.shape) == sz
+                        and t.device == self.sh.device and t.is_contiguous() and not t.is_conj() and not t.is_neg()
+                        for t, dt, sz in want)
+                and not torch.cuda.is_current_stream_capturing())
+
+    def _make_handle(self, ntheta):
+        h = ctypes.c_void_p()
+        _lib.call("ht_rec_create", self.n, self.nz, self.nobj, self.nzobj, ntheta, self.ndist,
+                  int(self.sh.obj_dtype == "complex64"), self.prop._h, ctypes.byref(h))
+        _lib.call("ht_rec_set_data_size", h, float(self.data_size))
+        _lib.call("ht_rec_set_zero_gradient", h, 1)   # torch.abs has gradient 0 at 0
+        return h
+
+    @contextlib.contextmanager
+    def handle(self, ntheta):
+        """A cascade handle for ntheta angles on the current stream."""
+        key = (ntheta, torch.cuda.current_stream(self.sh.device).cuda_stream)
+        with torch.cuda.device(self.sh.device):
+            h = self._handles.take(key, lambda: self._make_handle(ntheta))
+            try:
+                yield h
+            finally:
+                self._handles.put(key, h)
 
     def _term(self, proj, prb, pos, mag, data):
         out = proj.new_zeros((), dtype=torch.float32).real
@@ -156,6 +270,12 @@ class DataFidelity(torch.nn.Module):
         """F at (x, prb, pos): x is the object, or with proj=True the
         projections [ntheta, nzobj, nobj] (the BH variable proj)."""
         total = None
+        if self._use_fused(x, prb, pos, mag, data, proj):
+            for i, (a, b) in enumerate(self.bounds):
+                f = _ChunkMisfit.apply(x[a:b] if proj else x, prb, pos[a:b], mag[a:b], data[a:b], self,
+                                       None if proj else self.tomos[i])
+                total = f if total is None else total + f
+            return total
         for i, (a, b) in enumerate(self.bounds):
             args = (prb, pos[a:b], mag[a:b], data[a:b])
             if proj:

@@ -106,6 +106,7 @@ struct CascDims {
   int n, nz, nobj, nzobj, ndist;
   long nimg;         // ntheta * ndist
   int shared_c = 0;  // 1: one coefficient array [nzobj, nobj] for every angle
+  int zero_grad = 0; // 1: the gradient of |x0| at x0 = 0 is 0 (else x0 / |x0|, NaN there, as the reference has it)
 };
 
 // Offset of angle th's coefficient array.
@@ -395,7 +396,8 @@ k_casc_resid(float2* __restrict__ tmp, float2* __restrict__ x0c, const float* __
         if (MODE == 0) {
           x0c[row * N + tx] = x0;
           // rec_mpi.py:557-559: scale * (x - y * (x / |x|))
-          const float2 l = make_float2(x0.x / a, x0.y / a);
+          float2 l = make_float2(x0.x / a, x0.y / a);
+          if (D.zero_grad && a == 0.f) l = make_float2(0.f, 0.f);
           g0[i] = make_float2(scale * (x0.x - d * l.x), scale * (x0.y - d * l.y));
         }
       }
@@ -460,7 +462,8 @@ k_casc_resid512(float2* __restrict__ tmp, float2* __restrict__ x0c, const float*
       if (MODE == 0) {
         x0c[row * N + tx] = x0;
         // rec_mpi.py:557-559: scale * (x - y * (x / |x|))
-        const float2 l = make_float2(x0.x / a, x0.y / a);
+        float2 l = make_float2(x0.x / a, x0.y / a);
+          if (D.zero_grad && a == 0.f) l = make_float2(0.f, 0.f);
         v[i] = make_float2(scale * (x0.x - d * l.x), scale * (x0.y - d * l.y));
       }
     }
@@ -1404,6 +1407,13 @@ extern "C" int ht_rec_set_shared_coefficients(ht_rec_s* r, int shared) {
   using namespace ht;
   HT_REQUIRE(r, "ht_rec_set_shared_coefficients: null pointer");
   r->D.shared_c = shared ? 1 : 0;
+  return kOk;
+}
+
+extern "C" int ht_rec_set_zero_gradient(ht_rec_s* r, int on) {
+  using namespace ht;
+  HT_REQUIRE(r, "ht_rec_set_zero_gradient: null pointer");
+  r->D.zero_grad = on ? 1 : 0;
   return kOk;
 }
 

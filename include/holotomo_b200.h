@@ -230,6 +230,9 @@ int ht_rec_destroy(ht_rec_s* r);
 int ht_rec_forward(ht_rec_s* r, const void* c, const float* pos, const float* mag, const void* prb, const float* data,
                    float* amp, double* fval, void* stream);
 
+/* on = 1: the gradient of |x0| at x0 = 0 counts as 0 (torch.abs's rule); 0 (the
+ * default): x0 / |x0|, NaN there, as the reference has it (rec_mpi.py:557-559). */
+int ht_rec_set_zero_gradient(ht_rec_s* r, int on);
 /* A handle created for an angle chunk of a larger problem: N of the
  * objective's 2/N (rec_mpi.py:569, 91) becomes the whole problem's
  * ntheta*ndist*nz*n.  With it, ht_rec_gradient / ht_rec_hessian called on the

@@ -191,3 +191,38 @@ def test_autograd_matches_fused_cascade_at_256(ntheta, chunk):
     assert rel_l2((gprb * r["prb"]).cpu().numpy(), grads["prb"].cpu().numpy()) < 1e-4
     assert rel_l2((gpos * r["pos"]).cpu().numpy(), grads["pos"].cpu().numpy()) < 1e-4
     assert rel_l2((gobj * r["obj"]).cpu().numpy(), grads["obj"].cpu().numpy()) < 1e-4
+
+
+@pytest.mark.parametrize("n,nobj,obj_dtype,chunk", [(32, 48, "complex64", None), (64, 64, "complex64", 3),
+                                                    (64, 96, "float32", 4), (128, 256, "complex64", 5)])
+@pytest.mark.parametrize("proj", [False, True])
+def test_fidelity_fused_equals_operator_by_operator(n, nobj, obj_dtype, chunk, proj):
+    """The fused term against the composition of the single operators (which a
+    data gradient asks for): value and gradients, ragged chunks, object wider
+    than the detector, a distance whose probe is zero (|x0| has gradient 0 there)."""
+    from holotomocupy_b200.autograd import DataFidelity
+    rng = np.random.default_rng(n + nobj)
+    ntheta, ndist, nz = 7, 2, 64
+    theta = np.linspace(0, np.pi, ntheta, endpoint=False).astype("float32")
+    fid = DataFidelity.create(n, nz, nobj, nobj, theta, ndist, 7.3e-11, 20e-9, np.array([3e-3, 5e-3]), 0.9, chunk,
+                              obj_dtype)
+    shape = (ntheta, nobj, nobj) if proj else (nobj, nobj, nobj)
+    x = 0.05 * rng.standard_normal(shape).astype("float32")
+    if obj_dtype == "complex64":
+        x = (x + 0.01j * rng.standard_normal(shape)).astype("complex64")
+    prb = (1 + 0.1 * rng.standard_normal((ndist, nz, n)) + 0.1j).astype("complex64")
+    prb[1] = 0
+    pos = rng.uniform(-3, 3, (ntheta, ndist, 2)).astype("float32")
+    mag = rng.uniform(0.9, 1.0, (ntheta, ndist)).astype("float32")
+    data = (1 + 0.1 * rng.standard_normal((ntheta, ndist, nz, n))).astype("float32")
+    res = []
+    for fused in (True, False):
+        t = [cuda(a).requires_grad_() for a in (x, prb, pos)]
+        d = cuda(data).requires_grad_(not fused)
+        assert fid._use_fused(t[0], t[1], t[2], cuda(mag), d, proj) == fused
+        f = fid(*t, cuda(mag), d, proj=proj)
+        res.append([f.detach()] + list(torch.autograd.grad(2 * f, t)))
+    for a, b in zip(*res):
+        assert a.dtype == b.dtype and a.shape == b.shape
+        assert torch.isfinite(torch.view_as_real(a) if a.is_complex() else a).all()
+        assert rel_l2(a.cpu().numpy(), b.cpu().numpy()) < 1e-5, rel_l2(a.cpu().numpy(), b.cpu().numpy())
