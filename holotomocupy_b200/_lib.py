@@ -45,6 +45,7 @@ SIGNATURES = {
     "ht_shift_coeff": [_vp, _vp, _vp, _c_long, _vp],
     "ht_shift_coeffback": [_vp, _vp, _vp, _c_long, _c_float, _vp],
     "ht_shift_coeff_real": [_vp, _vp, _vp, _c_long, _vp],
+    "ht_shift_spline": [_vp, _vp, _vp, _c_long, _vp],
     "ht_shift_filter": [_vp, _vp, _vp, _c_long, _vp, _vp, _vp],
     "ht_shift_Sback": [_vp, _vp, _vp, _vp, ctypes.c_int, _vp, _c_long, _vp],
     "ht_shift_coeff_z": [_vp, _vp, _vp, _c_long, _vp],

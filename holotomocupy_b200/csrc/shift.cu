@@ -20,6 +20,7 @@
 #include "lines.cuh"
 #include "holotomo_b200_internal.h"
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -688,6 +689,32 @@ k_bspline_cols(const T* in, T* out, int n, long ncols, BsPole P) {
     if (k0 + k < n) out[(long)(k0 + k) * ncols + col] = u[k];
 }
 
+// The spline at the grid points, out = B c with B = (1, 4, 1) along both axes,
+// periodic: the prefilter's inverse.  A warp takes 32 columns of kSplineRows rows,
+// each row's sum along x formed once.
+constexpr int kSplineRows = 16, kSplineWarps = 8;
+__global__ void __launch_bounds__(32 * kSplineWarps)
+k_bspline_grid(const float2* __restrict__ c, float2* __restrict__ out, int ny, int nx) {
+  const int x = blockIdx.x * 32 + threadIdx.x, y0 = (blockIdx.y * kSplineWarps + threadIdx.y) * kSplineRows;
+  if (x >= nx || y0 >= ny) return;
+  const float2* src = c + (long)blockIdx.z * ny * nx;
+  float2* dst = out + (long)blockIdx.z * ny * nx + x;
+  const int xm = x == 0 ? nx - 1 : x - 1, xp = x + 1 == nx ? 0 : x + 1;
+  auto row = [&](int y) {
+    const float2* r = src + (long)y * nx;
+    const float2 a = __ldg(&r[xm]), b = __ldg(&r[x]), d = __ldg(&r[xp]);
+    return make_float2((a.x + d.x) + 4.f * b.x, (a.y + d.y) + 4.f * b.y);
+  };
+  float2 p = row(y0 == 0 ? ny - 1 : y0 - 1), q = row(y0);
+#pragma unroll 4
+  for (int y = y0; y < min(y0 + kSplineRows, ny); ++y) {
+    const float2 n = row(y + 1 == ny ? 0 : y + 1);
+    dst[(long)y * nx] = make_float2((p.x + n.x) + 4.f * q.x, (p.y + n.y) + 4.f * q.y);
+    p = q;
+    q = n;
+  }
+}
+
 template <class T>
 static cudaError_t bspline2d(const T* in, T* out, long batch, int ny, int nx, double b, cudaStream_t st) {
   constexpr int smem = kBsSpan * (kBsSpan + 1) * (int)sizeof(T);
@@ -990,6 +1017,25 @@ extern "C" int ht_shift_coeff_z(ht_shift_s* s, const void* in, void* out, long n
   HT_REQUIRE(ncols <= 0x7fffffffL, "ht_shift_coeff_z: ncols too large");
   HT_CHECK_CUDA(bspline_cols<float2>(static_cast<const float2*>(in), static_cast<float2*>(out), s->nzpsi, ncols,
                                      static_cast<cudaStream_t>(stream)));
+  return kOk;
+}
+
+extern "C" int ht_shift_spline(ht_shift_s* s, const void* c, void* out, long batch, void* stream) {
+  using namespace ht;
+  HT_REQUIRE(s && c && out, "ht_shift_spline: null pointer");
+  HT_REQUIRE(batch >= 0, "ht_shift_spline: batch must be non-negative");
+  const long img = (long)s->nzpsi * s->npsi;
+  const float2* src = static_cast<const float2*>(c);
+  float2* dst = static_cast<float2*>(out);
+  HT_REQUIRE(src + batch * img <= dst || dst + batch * img <= src, "ht_shift_spline: c and out must not overlap");
+  const int rows = kSplineRows * kSplineWarps;
+  for (long b = 0; b < batch; b += 65535) {
+    const dim3 grid((s->npsi + 31) / 32, (s->nzpsi + rows - 1) / rows, (unsigned)std::min(65535L, batch - b));
+    k_bspline_grid<<<grid, dim3(32, kSplineWarps), 0, static_cast<cudaStream_t>(stream)>>>(src + b * img, dst + b * img,
+                                                                                           s->nzpsi, s->npsi);
+    count_launch();
+    HT_CHECK_CUDA(cudaGetLastError());
+  }
   return kOk;
 }
 

@@ -221,7 +221,7 @@ class Rec:
         self._graph = None
         # BH keeps only the B-spline coefficients of proj up to date and applies
         # the prefilter as Cx inside R / R^T and Cz on the volume (complex
-        # objects); vars/grads/etas "proj" are recomputed by bh_finish()
+        # objects); bh_finish() forms vars/grads/etas "proj" from them
         self._fold = self.complex_obj
         # the folded (complex-object) iteration allocates nothing, so it may be
         # recorded into a CUDA graph
@@ -529,10 +529,12 @@ class Rec:
 
     def bh_finish(self):
         """End of BH (rec_mpi.py:229-232).  With the folded prefilter the proj
-        arrays, which are R of the obj arrays, are recomputed here."""
+        arrays are formed here from their B-spline coefficients, which the
+        iterations kept up to date."""
         if self._fold:
-            for d in (self.vars, self.grads, self.etas):
-                self.fwd_tomo(d["obj"], out=d["proj"])
+            for name, d in (("vars", self.vars), ("grads", self.grads), ("etas", self.etas)):
+                _lib.call("ht_shift_spline", self.cl_shift._hc, _lib.ptr(self._c[name]), _lib.ptr(d["proj"]),
+                          self.ntheta, _lib.stream_ptr())
         self.vars["obj"] *= self.norm_const
         return self.vars
 

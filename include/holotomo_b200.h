@@ -160,6 +160,10 @@ int ht_shift_coeff_real(ht_shift_s* s, const float* psi, float* out, long batch,
  * symbol 1 / ((4 + 2 b cos wy)(4 + 2 b cos wx)) with b = phi(1/m) in [0, 1]; complex64
  * [batch, nzpsi, npsi]; out must not overlap psi. */
 int ht_shift_coeffback(ht_shift_s* s, const void* psi, void* out, long batch, float b, void* stream);
+/* The prefilter's inverse: out[y, x] = the spline of coefficients c at the grid points,
+ * (1, 4, 1) along both axes, periodic; complex64 [batch, nzpsi, npsi]; out must not
+ * overlap c. */
+int ht_shift_spline(ht_shift_s* s, const void* c, void* out, long batch, void* stream);
 /* The z-axis half of the prefilter (the column factor of shift.py:74-82):
  * out = Cz in for in, out [nzpsi, ncols] complex64 (a volume [nzpsi, ny, nx]
  * has ncols = ny nx); out may alias in. */

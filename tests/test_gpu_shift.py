@@ -143,6 +143,9 @@ def test_prefilter_over_tiles(dtype, npsi, nzpsi):
         x = torch.from_numpy(psi).cuda()
         _lib.call("ht_shift_coeff", s._hc, _lib.ptr(x), _lib.ptr(x), 3, _lib.stream_ptr())
         assert rel_l2(x.cpu().numpy(), got.cpu().numpy()) < 1e-6
+        back = torch.empty_like(got)
+        _lib.call("ht_shift_spline", s._hc, _lib.ptr(got), _lib.ptr(back), 3, _lib.stream_ptr())
+        assert rel_l2(back.cpu().numpy(), psi) < 1e-6
         vol = torch.from_numpy(psi[0]).cuda()
         ref = np.fft.ifft(np.fft.fft(psi[0].astype(np.complex128), axis=0)
                           / (4 + 2 * np.cos(2 * np.pi * np.arange(nzpsi) / nzpsi))[:, None], axis=0)
