@@ -132,18 +132,45 @@ struct SmRow {
 };
 
 // Column line inside a [N][C] tile (row-major, C columns side by side).  For
-// C = 4 (32-byte rows) row k is stored at k ^ ((k >> 3) & 3): the rows 8
-// apart that the first radix-8 stage writes together then fall on different
-// banks, and consecutive rows stay on different banks.
+// C = 4 (32-byte rows) row k is stored at k ^ (g(k) & 3), g(k) = (k >> 3) ^ (k >> 4):
+// the rows 8 or 16 apart that the first stage of radix 8 or 16 writes together
+// then fall on different banks, and consecutive rows stay on different banks.
 template <int C>
 __host__ __device__ __forceinline__ int col_row(int k) {
-  return (C == 4) ? (k ^ ((k >> 3) & 3)) : k;
+  return (C == 4) ? (k ^ (((k >> 3) ^ (k >> 4)) & 3)) : k;
 }
 template <int C>
 struct SmCol {
   float2* p;  // points at column c of row 0
   __device__ __forceinline__ float2 ld(int k) const { return p[col_row<C>(k) * C]; }
   __device__ __forceinline__ void st(int k, float2 v) const { p[col_row<C>(k) * C] = v; }
+};
+
+// Column line with a spare row after every 2^SH rows, 2^SH being the first
+// stage's radix: for C = 8 (64-byte rows) the rows a radix apart that the first
+// stage writes together then fall on different banks.
+template <int C, int SH>
+struct SmColP {
+  float2* p;
+  static __host__ __device__ constexpr int padded(int n) { return n + (n >> SH); }
+  __device__ __forceinline__ float2 ld(int k) const { return p[(k + (k >> SH)) * C]; }
+  __device__ __forceinline__ void st(int k, float2 v) const { p[(k + (k >> SH)) * C] = v; }
+  __device__ __forceinline__ float2 ld_pad(int pk) const { return p[pk * C]; }
+  __device__ __forceinline__ void st_pad(int pk, float2 v) const { p[pk * C] = v; }
+};
+
+// Views with a spare slot after every 2^shift samples (-1: none).
+template <class V>
+struct pad_shift {
+  static constexpr int value = -1;
+};
+template <>
+struct pad_shift<SmRow> {
+  static constexpr int value = 4;
+};
+template <int C, int SH>
+struct pad_shift<SmColP<C, SH>> {
+  static constexpr int value = SH;
 };
 
 // --------------------------------------------------------------- the plan
@@ -171,9 +198,9 @@ HT_PLAN(36, 12, 4, 3, 3)
 HT_PLAN(48, 12, 4, 4, 3)
 HT_PLAN(64, 8, 8, 8)
 HT_PLAN(96, 24, 8, 4, 3)
-HT_PLAN(128, 8, 8, 4, 4)
+HT_PLAN(128, 16, 16, 8)
 HT_PLAN(192, 24, 8, 8, 3)
-HT_PLAN(256, 8, 8, 8, 4)
+HT_PLAN(256, 16, 16, 16)
 HT_PLAN(384, 12, 4, 4, 4, 3, 2)   // 12 samples a thread: the stencil row kernels keep their occupancy
 HT_PLAN(512, 8, 8, 8, 8)
 HT_PLAN(768, 12, 4, 4, 4, 4, 3)
@@ -199,12 +226,18 @@ struct ColPlan<768> : PlanOf<768, 24, 8, 8, 4, 3> {};
 // rows carry the stencil work beside the transform (so more threads a line
 // pay): the row plan, except at 1024 samples, where 8 samples a thread (128
 // threads a line) beat 16 (BH iteration at 1024^2 x 256 x 4: 273 against
-// 283 ms); the other 1024-sample lines (the Radon transform's at n = 512)
-// keep 16, which is faster for them.
+// 283 ms; the other 1024-sample lines, the Radon transform's at n = 512, keep
+// 16, which is faster for them), and at 128 and 256, which keep 8 where the
+// column and residual passes take 16 in two radix-16 stages (720 images of
+// 128^2: column pass 106 us to 92, residual pass 117 to 98).
 template <int N>
 struct StPlan : Plan<N> {};
 template <>
 struct StPlan<1024> : PlanOf<1024, 8, 8, 8, 8, 2> {};
+template <>
+struct StPlan<256> : PlanOf<256, 8, 8, 8, 4> {};
+template <>
+struct StPlan<128> : PlanOf<128, 8, 8, 4, 4> {};
 
 // ------------------------------------------------------ synchronisation
 // Barrier between the stages of one line's transform.  CtaSync: the whole
@@ -280,6 +313,8 @@ struct SplitView {
   S s;
   __device__ __forceinline__ float2 ld(int k) const { return l.ld(k); }
   __device__ __forceinline__ void st(int k, float2 v) const { s.st(k, v); }
+  __device__ __forceinline__ float2 ld_pad(int pk) const { return l.ld_pad(pk); }
+  __device__ __forceinline__ void st_pad(int pk, float2 v) const { s.st_pad(pk, v); }
 };
 
 // A view of a zero-padded line declares kCentralHalf: only its samples N/4 <= k <
@@ -301,6 +336,17 @@ struct store_half : central_half<V> {};
 template <class L, class S>
 struct store_half<SplitView<L, S>> : central_half<S> {};
 
+// The padded side of a stage's view, if its loads (stores) go through one.
+template <class V>
+struct load_pad : pad_shift<V> {};
+template <class L, class S>
+struct load_pad<SplitView<L, S>> : pad_shift<L> {};
+template <class V>
+struct store_pad : pad_shift<V> {};
+template <class L, class S>
+struct store_pad<SplitView<L, S>> : pad_shift<S> {};
+__host__ __device__ constexpr int max0(int x) { return x > 0 ? x : 0; }
+
 // ------------------------------------------------------------- one stage
 // tw4: table of exp(-2 pi i m / (4N)); W_N^a = tw4[4a].  SYNC_MID: barrier
 // between the loads and the stores (needed when both are the same shared
@@ -317,10 +363,11 @@ __device__ __forceinline__ void fft_stage(float2 (&v)[E], const SM& sm, int t,
 #pragma unroll
   for (int s = 0; s < NB; ++s) {
     const int b = t + s * T;
-    if constexpr (std::is_same<SM, SmRow>::value && NR % 16 == 0) {
-      const int pb = b + (b >> 4);
+    if constexpr (load_pad<SM>::value >= 0 && NR % (1 << max0(load_pad<SM>::value)) == 0) {
+      constexpr int SH = max0(load_pad<SM>::value);
+      const int pb = b + (b >> SH);
 #pragma unroll
-      for (int j = 0; j < R; ++j) v[s * R + j] = sm.ld_pad(pb + j * (NR + NR / 16));
+      for (int j = 0; j < R; ++j) v[s * R + j] = sm.ld_pad(pb + j * (NR + (NR >> SH)));
     } else {
 #pragma unroll
       for (int j = 0; j < R; ++j) {
@@ -351,11 +398,15 @@ __device__ __forceinline__ void fft_stage(float2 (&v)[E], const SM& sm, int t,
   for (int s = 0; s < NB; ++s) {
     const int b = t + s * T;
     const int i = (P > 1) ? (b % P) : 0;
-    if constexpr (std::is_same<SM, SmRow>::value && P % 16 == 0) {
+    constexpr int SH = max0(store_pad<SM>::value);
+    if constexpr (store_pad<SM>::value >= 0 && P % (1 << SH) == 0) {
       const int k0 = (b - i) * R + i;
-      const int pk = k0 + (k0 >> 4);
+      const int pk = k0 + (k0 >> SH);
 #pragma unroll
-      for (int j = 0; j < R; ++j) sm.st_pad(pk + j * (P + P / 16), v[s * R + j]);
+      for (int j = 0; j < R; ++j) sm.st_pad(pk + j * (P + (P >> SH)), v[s * R + j]);
+    } else if constexpr (store_pad<SM>::value >= 0 && P == 1 && R == (1 << SH)) {
+#pragma unroll
+      for (int j = 0; j < R; ++j) sm.st_pad(b * (R + 1) + j, v[s * R + j]);
     } else {
 #pragma unroll
       for (int j = 0; j < R; ++j) {

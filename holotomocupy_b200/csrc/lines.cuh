@@ -6,9 +6,9 @@
 namespace ht {
 
 // Rows per CTA for a row pass of length N: about 256 threads per CTA.
-template <int N>
+template <int N, class PL = Plan<N>>
 struct RowCfg {
-  static constexpr int T = Plan<N>::T;
+  static constexpr int T = PL::T;
   static constexpr int LINES = (T >= 256) ? 1 : (256 / T);
   static constexpr int THREADS = LINES * T;
   static constexpr int SMEM = LINES * SmRow::padded(N) * (int)sizeof(float2);
@@ -17,12 +17,14 @@ struct RowCfg {
 };
 
 // Columns per CTA for a column pass of length N (tile N x C in shared memory;
-// at N >= 2048 the 4-column tile's rows are swizzled, see SmCol).
+// the 4-column tile's rows at N >= 3072 are swizzled, see SmCol).  At 2048 samples
+// eight columns and 1024 threads beat four and two CTAs per SM: D at 2048^2 x 16
+// images 1.21 ms against 1.27.
 template <int N>
 struct ColCfg {
   using PL = ColPlan<N>;
   static constexpr int T = PL::T;
-  static constexpr int C = (N >= 2048) ? 4 : ((N >= 256) ? 8 : 16);
+  static constexpr int C = (N >= 3072) ? 4 : ((N >= 256) ? 8 : 16);
   static constexpr int THREADS = C * T;
   static constexpr int SMEM = N * C * (int)sizeof(float2);
   // two CTAs per SM where that leaves 64 registers a thread (one CTA's block

@@ -45,20 +45,32 @@ struct RowOut {
   }
 };
 
+// The row passes' plan: the row plan, but 8 samples a thread at 128 and 256,
+// where a few small images leave the chip idle and more threads a line shorten
+// their passes: D of 17 images of 128^2 12.5 us against 13.7 with 16 samples, of
+// 256 x 64 10.9 against 12.3; 24 images of 256^2 31.5 against 29.8.  (One plan
+// for every number of images: an image's samples do not depend on its batch.)
+template <int N>
+struct StRowPlan : Plan<N> {};
+template <>
+struct StRowPlan<128> : StPlan<128> {};
+template <>
+struct StRowPlan<256> : StPlan<256> {};
+
 // in, out: [nrows, N]; out may alias in (a line's loads come before its first
 // store).  The first FFT stage loads from global memory, the output combine
 // stores there: a sample passes shared memory between the stages only.
 template <int N>
-__global__ void __launch_bounds__(RowCfg<N>::THREADS)
+__global__ void __launch_bounds__(RowCfg<N, StRowPlan<N>>::THREADS)
 k_dct2_rows(const float2* in, float2* out, long nrows, const float2* __restrict__ tw4) {
-  constexpr int T = RowCfg<N>::T;
+  constexpr int T = RowCfg<N, StRowPlan<N>>::T;
   constexpr int LS = SmRow::padded(N);
   extern __shared__ float2 smem[];
   const int line = threadIdx.x / T, t = threadIdx.x % T;
-  const long row = (long)blockIdx.x * RowCfg<N>::LINES + line;
+  const long row = (long)blockIdx.x * RowCfg<N, StRowPlan<N>>::LINES + line;
   const bool valid = row < nrows;
   SmRow sm{smem + line * LS};
-  fft_line_from<N, false>(RowIn<N>{in + (valid ? row : nrows - 1) * N}, sm, t, tw4, line_sync<T>());
+  fft_line_from<N, false, StRowPlan<N>>(RowIn<N>{in + (valid ? row : nrows - 1) * N}, sm, t, tw4, line_sync<T>());
   if (!valid) return;
   float2* dst = out + row * N;
 #pragma unroll
@@ -77,13 +89,13 @@ k_dct2_rows(const float2* in, float2* out, long nrows, const float2* __restrict_
 // The combine loads a line's samples in pairs, all before its first store; the
 // last FFT stage stores to global memory.
 template <int N>
-__global__ void __launch_bounds__(RowCfg<N>::THREADS)
+__global__ void __launch_bounds__(RowCfg<N, StRowPlan<N>>::THREADS)
 k_dct3_rows(const float2* in, float2* out, long nrows, const float2* __restrict__ tw4) {
-  constexpr int T = RowCfg<N>::T;
+  constexpr int T = RowCfg<N, StRowPlan<N>>::T;
   constexpr int LS = SmRow::padded(N);
   extern __shared__ float2 smem[];
   const int line = threadIdx.x / T, t = threadIdx.x % T;
-  const long row = (long)blockIdx.x * RowCfg<N>::LINES + line;
+  const long row = (long)blockIdx.x * RowCfg<N, StRowPlan<N>>::LINES + line;
   const bool valid = row < nrows;
   SmRow sm{smem + line * LS};
   const float2* src = in + (valid ? row : nrows - 1) * N;
@@ -109,7 +121,7 @@ k_dct3_rows(const float2* in, float2* out, long nrows, const float2* __restrict_
     }
   }
   line_sync<T>()();
-  fft_line_to<N, false>(sm, RowOut<N>{out + row * N, valid}, t, tw4, line_sync<T>());
+  fft_line_to<N, false, StRowPlan<N>>(sm, RowOut<N>{out + row * N, valid}, t, tw4, line_sync<T>());
 }
 
 // Rows of 512 samples, a warp a row, on the register transforms of row512.cuh:
@@ -170,10 +182,8 @@ struct ColOut {
 // the last one stores them there (a warp covers 32/C rows of C adjacent
 // columns per access), so the column tile passes through shared memory only
 // between stages.
-// Two CTAs per SM up to 512 threads (ColCfg::MIN_BLOCKS; the register cap
-// this sets, 64, spills a little at NZ = 2048): the block barriers of one CTA
-// overlap the other's work (D at 2048^2 x 16 images 1.88 -> 1.67 ms, at
-// 1024^2 x 32 0.80 -> 0.72 ms).
+// Two CTAs per SM up to 512 threads (ColCfg::MIN_BLOCKS): the block barriers of
+// one CTA overlap the other's work (D at 1024^2 x 32 0.80 -> 0.72 ms).
 template <int NZ, bool CONJ>
 __global__ void __launch_bounds__(ColCfg<NZ>::THREADS, ColCfg<NZ>::MIN_BLOCKS)
 k_dct_cols(float2* data, int n, const float2* __restrict__ Hall, int ntab, const float2* __restrict__ tw4) {
@@ -218,10 +228,13 @@ k_dct_cols(float2* data, int n, const float2* __restrict__ Hall, int ntab, const
 // samples k = b + 64 j are closed under k -> 512 - k.  The k / N-k combine,
 // the table product and the DCT-III pre-combine of both samples of a pair
 // then happen in registers, so the spectrum makes no round trip through
-// shared memory between the two transforms.
+// shared memory between the two transforms.  The tile has a spare row after
+// every eight (SmColP: without it the first stage's stores meet on the banks;
+// 900 images of 512^2 1.84 -> 1.78 ms).
 struct Col512 {
   static constexpr int N = 512, E = 16, T = 32, C = 8, THREADS = C * T;
-  static constexpr int SMEM = N * C * (int)sizeof(float2);
+  using SM = SmColP<C, 3>;
+  static constexpr int SMEM = SM::padded(N) * C * (int)sizeof(float2);
 };
 
 // DCT-II output pair (X[k], X[N-k]) -> x Hw -> DCT-III input pair, 0 < k < N/2
@@ -253,11 +266,11 @@ k_dct_cols512(float2* data, int n, const float2* __restrict__ Hall, int ntab, co
   const int col = min((int)blockIdx.x * C + c, n - 1);
   const float2* __restrict__ H = H0 + col;
   float2* img = data + (long)blockIdx.y * N * n + col;
-  SmCol<C> sm{tile + c};
+  const Col512::SM sm{tile + c};
   const CtaSync sync{};
   float2 v[E];
   // DCT-II FFT: stages 1 (from global memory) and 2
-  fft_stage<N, E, 8, 1, false, false, true>(v, SplitView<ColIn<N>, SmCol<C>>{ColIn<N>{img, n, valid}, sm}, t, tw4,
+  fft_stage<N, E, 8, 1, false, false, true>(v, SplitView<ColIn<N>, Col512::SM>{ColIn<N>{img, n, valid}, sm}, t, tw4,
                                             sync);
   fft_stage<N, E, 8, 8, false, true, true>(v, sm, t, tw4, sync);
   // stage 3 (P = 64) for the butterflies b0, b1, kept in registers: v[8 s + j] = X[b_s + 64 j]
@@ -266,7 +279,7 @@ k_dct_cols512(float2* data, int n, const float2* __restrict__ Hall, int ntab, co
   for (int s = 0; s < 2; ++s) {
     const int b = s ? b1 : b0;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[8 * s + j] = sm.ld(b + 64 * j);
+    for (int j = 0; j < 8; ++j) v[8 * s + j] = sm.ld_pad(b + (b >> 3) + 72 * j);
     float2 w[8];
     twiddles<8, false>(tw4, b, N, w);
 #pragma unroll
@@ -308,11 +321,11 @@ k_dct_cols512(float2* data, int n, const float2* __restrict__ Hall, int ntab, co
     const int b = s ? b1 : b0;
     Dft<8, false>::run(&v[8 * s]);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) sm.st(b * 8 + j, v[8 * s + j]);
+    for (int j = 0; j < 8; ++j) sm.st_pad(b * 9 + j, v[8 * s + j]);
   }
   sync();
   fft_stage<N, E, 8, 8, false, true, true>(v, sm, t, tw4, sync);
-  fft_stage<N, E, 8, 64, false, false, false>(v, SplitView<SmCol<C>, ColOut<N>>{sm, ColOut<N>{img, n, valid}}, t,
+  fft_stage<N, E, 8, 64, false, false, false>(v, SplitView<Col512::SM, ColOut<N>>{sm, ColOut<N>{img, n, valid}}, t,
                                               tw4, sync);
 }
 
@@ -326,7 +339,7 @@ static cudaError_t launch_dct_rows(bool inverse, const float2* in, float2* out, 
     ::ht::count_launch();
     return cudaGetLastError();
   }
-  using CF = RowCfg<N>;
+  using CF = RowCfg<N, StRowPlan<N>>;
   const long grid = (nrows + CF::LINES - 1) / CF::LINES;
   if (inverse) {
     cudaError_t e = allow_smem(k_dct3_rows<N>, CF::SMEM);
