@@ -152,12 +152,33 @@ struct RowGeo {
   }
 };
 
-// Horizontal stencil of one detector pixel (same conventions).
+// Horizontal stencil of one detector pixel: its four taps' first position in
+// the vertically reduced rows, which have kVPad zeros on either side of the
+// object, so that no tap is tested against the object's edges.
+constexpr int kVPad = 4;
 template <int ORDER>
 struct ColGeo {
-  int xx[4];
+  int x0;
   float px[4], dpx[4], d2px[4];
   __device__ __forceinline__ ColGeo(const CascDims& D, float mag, float rx, int tx) {
+    const float x = sample_x(D, mag, rx, tx);
+    const float fx = floorf(x);
+    const float dx = x - fx;
+    bw0(dx, px);
+    if (ORDER >= 1) bw1(dx, dpx);
+    if (ORDER >= 2) bw2(dx, d2px);
+    x0 = (int)fminf(fmaxf(fx - 1.0f, -(float)kVPad), (float)D.nobj) + kVPad;
+  }
+};
+
+// The same with the edges tested per tap (taps outside the object: column 0,
+// weight 0), for the Hessian row pass, whose rows have no margins: 5.0 ms against
+// 5.4 for 900 images of 512^2 in both directions.
+template <int ORDER>
+struct ColGeoEdge {
+  int xx[4];
+  float px[4], dpx[4], d2px[4];
+  __device__ __forceinline__ ColGeoEdge(const CascDims& D, float mag, float rx, int tx) {
     const float x = sample_x(D, mag, rx, tx);
     const int ix = (int)floorf(x);
     const float dx = x - (float)ix;
@@ -217,8 +238,8 @@ struct StCfg {
   static_assert(T % 32 != 0 || LINES * NFFT <= 15, "at most 15 line barriers per block");
   // dynamic shared memory: FFT lines, then reduction scratch, then the rows
   static constexpr int FFT_BYTES = LINES * NFFT * SmRow::padded(N) * 8;
-  static int bytes(int K, int nobj, int elem) {
-    return FFT_BYTES + red_doubles<TR>(K, THREADS) * 8 + LINES * NSET * nobj * elem;
+  static int bytes(int K, int nobj, int elem, int pad = 0) {
+    return FFT_BYTES + red_doubles<TR>(K, THREADS) * 8 + LINES * NSET * (nobj + pad) * elem;
   }
 };
 
@@ -241,16 +262,19 @@ __device__ __forceinline__ void vrows(T* __restrict__ V, int nobj, const T* __re
       El<T>::fma(a, w[k][1], v1);
       El<T>::fma(a, w[k][2], v2);
       El<T>::fma(a, w[k][3], v3);
-      V[k * nobj + ix] = a;
+      V[k * (nobj + 2 * kVPad) + kVPad + ix] = a;
     }
   }
+  for (int i = t; i < 2 * kVPad; i += TT)
+#pragma unroll
+    for (int k = 0; k < NS; ++k) V[k * (nobj + 2 * kVPad) + (i < kVPad ? i : nobj + i)] = El<T>::zero();
 }
 
 // the four samples of a vertically reduced row under a pixel's stencil
 template <class T>
-__device__ __forceinline__ void vrow4(const T* __restrict__ V, const int (&xx)[4], T (&v)[4]) {
+__device__ __forceinline__ void vrow4(const T* __restrict__ V, int x0, T (&v)[4]) {
 #pragma unroll
-  for (int j = 0; j < 4; ++j) v[j] = V[xx[j]];
+  for (int j = 0; j < 4; ++j) v[j] = V[x0 + j];
 }
 
 // Two adjacent elements of T moved as one vector (16 bytes for complex, 8 for
@@ -332,7 +356,7 @@ k_casc_fwd(const T* __restrict__ c, const float* __restrict__ pos, const float* 
   const int k = (int)(img % D.ndist);
   const long th = img / D.ndist;
   SmRow sm{smem + line * SmRow::padded(N)};
-  T* V = reinterpret_cast<T*>(reinterpret_cast<char*>(smem) + CF::FFT_BYTES) + (long)line * D.nobj;
+  T* V = reinterpret_cast<T*>(reinterpret_cast<char*>(smem) + CF::FFT_BYTES) + (long)line * (D.nobj + 2 * kVPad);
   const float m0 = valid ? mag[img] : 1.f;
   const float2 r = valid ? ld_pos(pos, img) : make_float2(0.f, 0.f);
   const RowGeo<0> rg(D, m0, r.x, ty);
@@ -346,7 +370,7 @@ k_casc_fwd(const T* __restrict__ c, const float* __restrict__ pos, const float* 
     if (valid) {
       const ColGeo<0> cg(D, m0, r.y, tx);
       T v[4];
-      vrow4(V, cg.xx, v);
+      vrow4(V, cg.x0, v);
       const T x22 = dot4(cg.px, v);
       u = cmul(prb[((long)k * D.nz + ty) * N + tx], cexp_i(El<T>::cplx(x22)));
     }
@@ -556,8 +580,9 @@ __device__ __forceinline__ void cand_range(float m0, float C0, int i, int nhalf,
 }
 
 // cand_range with the reciprocal rm0 = 1 / m0 computed once (0 when
-// |m0| <= 1e-3: every index is a candidate).  The quotient moves by an ulp at
-// most, well inside the one-index margin on either side.
+// |m0| <= 1e-3: every index is a candidate), and no wider than the rounding of
+// the positions asks for: coordinates up to 4096 carry an error below 1e-3, so
+// a pixel's index one below 1e-3 |rm0| + 1e-3.  About 4 |rm0| + 1 candidates.
 __device__ __forceinline__ float cand_rm0(float m0) { return (fabsf(m0) > 1e-3f) ? 1.0f / m0 : 0.f; }
 __device__ __forceinline__ void cand_range_r(float rm0, float C0, int i, int nhalf, int nmax, int& lo, int& hi) {
   if (rm0 == 0.f) {
@@ -567,23 +592,24 @@ __device__ __forceinline__ void cand_range_r(float rm0, float C0, int i, int nha
   }
   const float a = ((float)(i - 2) - C0) * rm0 + (float)nhalf;
   const float b = ((float)(i + 2) - C0) * rm0 + (float)nhalf;
-  const float l = fminf(fmaxf(fminf(a, b), -1e7f), 1e7f);
-  const float h = fminf(fmaxf(fmaxf(a, b), -1e7f), 1e7f);
-  lo = max(0, (int)floorf(l) - 1);
-  hi = min(nmax - 1, (int)ceilf(h) + 1);
+  const float e = 0.01f + 0.002f * fabsf(rm0);
+  const float l = fminf(fmaxf(fminf(a, b) - e, -1e7f), 1e7f);
+  const float h = fminf(fmaxf(fmaxf(a, b) + e, -1e7f), 1e7f);
+  lo = max(0, (int)ceilf(l));
+  hi = min(nmax - 1, (int)floorf(h));
 }
 
 // The adjoint's horizontal gather reads, per detector pixel, the first object
 // column of its stencil (int) and its four tap weights (float): 20 bytes, kept
 // where the vertically reduced rows were once those are consumed.  Elements of
 // T per detector row of that shared area:
-// The vertical rows themselves: set 0 as nobj elements, then sets 1 and 2
-// as nobj pairs from an even offset (so that a pair loads as one vector).
+// The vertical rows themselves: set 0 as nobj + 2 kVPad elements, then sets 1 and
+// 2 as pairs from an even offset (so that a pair loads as one vector).
 constexpr int kAdjTabBytes = 20;
-__host__ __device__ constexpr int adj_pair_off(int nobj) { return (nobj + 1) / 2 * 2; }
+__host__ __device__ constexpr int adj_pair_off(int nobj) { return (nobj + 2 * kVPad + 1) / 2 * 2; }
 __host__ __device__ constexpr int adj_line_elems(int nobj, int n, int elem) {
-  return ((adj_pair_off(nobj) + 2 * nobj) * elem >= kAdjTabBytes * n)
-             ? adj_pair_off(nobj) + 2 * nobj
+  return ((adj_pair_off(nobj) + 2 * (nobj + 2 * kVPad)) * elem >= kAdjTabBytes * n)
+             ? adj_pair_off(nobj) + 2 * (nobj + 2 * kVPad)
              : ((kAdjTabBytes * n + elem - 1) / elem + 1) / 2 * 2;
 }
 
@@ -608,8 +634,13 @@ __device__ __forceinline__ void vrows_adj(T* __restrict__ V0, T* __restrict__ V1
       El<T>::fma(a[k], w[k][2], v2);
       El<T>::fma(a[k], w[k][3], v3);
     }
-    V0[ix] = a[0];
-    Pair<T>::st(V12 + 2 * ix, a[1], a[2]);
+    V0[kVPad + ix] = a[0];
+    Pair<T>::st(V12 + 2 * (kVPad + ix), a[1], a[2]);
+  }
+  for (int i = t; i < 2 * kVPad; i += TT) {
+    const int at = i < kVPad ? i : nobj + i;
+    V0[at] = El<T>::zero();
+    Pair<T>::st(V12 + 2 * at, El<T>::zero(), El<T>::zero());
   }
 }
 
@@ -662,9 +693,9 @@ k_casc_adj(const float2* __restrict__ tmp, float2* __restrict__ Pc, T* __restric
     T ay = El<T>::zero(), hxy = El<T>::zero(), hyy = El<T>::zero();
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const T a0 = V0[cg.xx[j]];
+      const T a0 = V0[cg.x0 + j];
       T a1, a2;
-      Pair<T>::ld(V12 + 2 * cg.xx[j], a1, a2);
+      Pair<T>::ld(V12 + 2 * (cg.x0 + j), a1, a2);
       El<T>::fma(x22, cg.px[j], a0);
       El<T>::fma(ax, cg.dpx[j], a0);
       El<T>::fma(hxx, cg.d2px[j], a0);
@@ -729,20 +760,36 @@ k_casc_adj(const float2* __restrict__ tmp, float2* __restrict__ Pc, T* __restric
 }
 
 // ================================================= probe gradient
-// gprb[k, p] = sum_theta P[theta, k, p]  (gF1, rec_mpi.py:641)
-__global__ void k_sum_theta(const float2* __restrict__ Pc, float2* __restrict__ gprb, long ntheta, int ndist,
-                            long npix, float scale, int acc) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;  // k * npix + p
-  if (i >= (long)ndist * npix) return;
-  const int k = (int)(i / npix);
-  const long p = i % npix;
+// gprb[k, p] = sum_theta P[theta, k, p]  (gF1, rec_mpi.py:641).  A block takes
+// kSumPix pixels; its kSumParts groups of threads each sum a contiguous part of
+// the angles, so that a small detector's few pixels still keep enough loads in
+// flight (720 images of 128^2: 66 us with a thread a pixel).
+constexpr int kSumPix = 64, kSumParts = 4;
+__global__ void __launch_bounds__(kSumPix * kSumParts)
+k_sum_theta(const float2* __restrict__ Pc, float2* __restrict__ gprb, long ntheta, int ndist, long npix, float scale,
+            int acc) {
+  __shared__ double2 part[kSumParts][kSumPix];
+  const long i = (long)blockIdx.x * kSumPix + threadIdx.x;  // k * npix + p
+  const bool valid = i < (long)ndist * npix;
+  const int k = valid ? (int)(i / npix) : 0;
+  const long p = valid ? i % npix : 0;
+  const long per = (ntheta + kSumParts - 1) / kSumParts;
+  const long th0 = threadIdx.y * per, th1 = min(th0 + per, ntheta);
   double sx = 0.0, sy = 0.0;
   // unrolled: the loads of eight angles are in flight, the sums keep angle order
 #pragma unroll 8
-  for (long th = 0; th < ntheta; ++th) {
+  for (long th = th0; th < th1; ++th) {
     const float2 v = Pc[(th * ndist + k) * npix + p];
     sx += v.x;
     sy += v.y;
+  }
+  part[threadIdx.y][threadIdx.x] = make_double2(sx, sy);
+  __syncthreads();
+  if (threadIdx.y != 0 || !valid) return;
+#pragma unroll
+  for (int j = 1; j < kSumParts; ++j) {
+    sx += part[j][threadIdx.x].x;
+    sy += part[j][threadIdx.x].y;
   }
   // the float sum times the variable scaling (rec_mpi.py:345: y[0] * rho_sq['prb'])
   const float2 g = make_float2((float)sx * scale, (float)sy * scale);
@@ -775,6 +822,7 @@ k_casc_vsum(T* __restrict__ gc, const T* __restrict__ hbuf, const float* __restr
   for (int r = 0; r < kVRows; ++r) acc[r] = El<T>::zero();
   for (int k = 0; k < D.ndist; ++k) {
     const long img = th * D.ndist + k;
+    if (img >= D.nimg) break;  // the last group of a shared array's images
     const float m0 = mag[img];
     const float ry = pos[2 * img + 0];
     const float C0 = -ry + (m0 - 1.0f) / 2.0f + (float)(D.nzobj / 2);
@@ -802,6 +850,21 @@ k_casc_vsum(T* __restrict__ gc, const T* __restrict__ hbuf, const float* __restr
 #pragma unroll
   for (int r = 0; r < kVRows; ++r)
     if (iy0 + r < D.nzobj) gc[(th * D.nzobj + iy0 + r) * D.nobj + ix] = acc[r];
+}
+
+// gc[i] = sum over groups g of part[g][i] (in order, in double precision)
+template <class T>
+__global__ void k_vsum_groups(const T* __restrict__ part, T* __restrict__ gc, long n, int groups) {
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double sx = 0.0, sy = 0.0;
+#pragma unroll 8
+  for (int g = 0; g < groups; ++g) {
+    const float2 v = El<T>::cplx(part[g * n + i]);
+    sx += v.x;
+    sy += v.y;
+  }
+  gc[i] = El<T>::from_sm(make_float2((float)sx, (float)sy));
 }
 
 // gpos[img] = (-Ay, -Ax)  (dsadj, cuda_kernels.py:744-761 with redot)
@@ -870,7 +933,7 @@ k_casc_hess_fwd(const T* __restrict__ c, const float* __restrict__ pos, const fl
     const float2 P = Pnext;
     if (valid && tx + TT < N) Pnext = Prow[tx + TT];
     if (valid) {
-      const ColGeo<1> cg(D, m0, r.y, tx);
+      const ColGeoEdge<1> cg(D, m0, r.y, tx);
       // the horizontal taps: every set of one tap's column in NS / 2 vector loads
       T x22 = El<T>::zero(), dxc = El<T>::zero(), dyc = El<T>::zero();
       T s0 = El<T>::zero(), ax0 = El<T>::zero(), ay0 = El<T>::zero();
@@ -1211,8 +1274,8 @@ namespace ht {
 // Dynamic shared memory of the stencil row kernels, checked against the device
 // limit (the vertically reduced rows grow with nobj).
 template <class CF>
-static cudaError_t stencil_smem(const void* kernel, int K, int nobj, int elem, int* bytes) {
-  *bytes = CF::bytes(K, nobj, elem);
+static cudaError_t stencil_smem(const void* kernel, int K, int nobj, int elem, int* bytes, int pad = 0) {
+  *bytes = CF::bytes(K, nobj, elem, pad);
   if (*bytes > 227 * 1024) {
     set_error("fused cascade: nobj = " + std::to_string(nobj) + " needs " + std::to_string(*bytes) +
               " bytes of shared memory per block (limit 227 KB)");
@@ -1239,7 +1302,7 @@ static cudaError_t launch_fwd(const CascDims& D, const T* c, const float* pos, c
                               float2* tmp, const float2* twn, cudaStream_t st) {
   using CF = StCfg<N, 1, 1>;
   int smem = 0;
-  cudaError_t e = stencil_smem<CF>(nullptr, 0, D.nobj, (int)sizeof(T), &smem);
+  cudaError_t e = stencil_smem<CF>(nullptr, 0, D.nobj, (int)sizeof(T), &smem, 2 * kVPad);
   if (e == cudaSuccess) e = allow_smem(k_casc_fwd<N, T>, smem);
   if (e != cudaSuccess) return e;
   const long nrows = D.nimg * D.nz;
@@ -1312,16 +1375,27 @@ static cudaError_t grad_impl(ht_rec_s* r, const void* c, const float* pos, const
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if ((e = reduce_rows(r, 5, kAx, 0, 5, 0, 0, st)) != cudaSuccess) return e;
   const long npix = (long)r->D.nz * N;
-  k_sum_theta<<<(unsigned)((r->D.ndist * npix + 255) / 256), 256, 0, st>>>(r->P, gprb, r->ntheta, r->D.ndist, npix,
-                                                                             sprb, acc);
+  k_sum_theta<<<(unsigned)((r->D.ndist * npix + kSumPix - 1) / kSumPix), dim3(kSumPix, kSumParts), 0, st>>>(
+      r->P, gprb, r->ntheta, r->D.ndist, npix, sprb, acc);
   ::ht::count_launch();
   if (r->D.shared_c) {
-    // one coefficient array for all angles: its gradient sums every image
-    // (all images taken as the distances of a single angle)
-    CascDims all = r->D;
-    all.ndist = (int)r->D.nimg;
-    dim3 g1((r->D.nobj + 31) / 32, (r->D.nzobj + 8 * kVRows - 1) / (8 * kVRows), 1);
-    k_casc_vsum<T><<<g1, dim3(32, 8), 0, st>>>((T*)gc, hbuf, pos, mag, all);
+    // one coefficient array for all angles: its gradient sums every image.  The
+    // images go in groups (each taken as the distances of one angle), whose sums
+    // lie in the consumed spectra and are added afterwards: one array's columns
+    // alone are too few threads (96 images of 512^2 on 768^2: 607 us).
+    const long narr = (long)r->D.nzobj * r->D.nobj;
+    const long room = nrows * N * (long)sizeof(float2) / (narr * (long)sizeof(T));
+    const int want = (int)std::max(1L, std::min({32L, room, r->D.nimg}));
+    CascDims part = r->D;
+    part.ndist = (int)((r->D.nimg + want - 1) / want);
+    const int groups = (int)((r->D.nimg + part.ndist - 1) / part.ndist);
+    T* sums = groups > 1 ? reinterpret_cast<T*>(r->tmp) : (T*)gc;
+    dim3 g1((r->D.nobj + 31) / 32, (r->D.nzobj + 8 * kVRows - 1) / (8 * kVRows), groups);
+    k_casc_vsum<T><<<g1, dim3(32, 8), 0, st>>>(sums, hbuf, pos, mag, part);
+    if (groups > 1) {
+      ::ht::count_launch();
+      k_vsum_groups<T><<<(unsigned)((narr + 255) / 256), 256, 0, st>>>(sums, (T*)gc, narr, groups);
+    }
   } else {
     dim3 g2((r->D.nobj + 31) / 32, (r->D.nzobj + 8 * kVRows - 1) / (8 * kVRows), r->ntheta);
     k_casc_vsum<T><<<g2, dim3(32, 8), 0, st>>>((T*)gc, hbuf, pos, mag, r->D);
