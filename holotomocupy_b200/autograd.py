@@ -123,8 +123,8 @@ class _ChunkMisfit(torch.autograd.Function):
                       _lib.stream_ptr())
         gx = None
         if ctx.needs_input_grad[0]:
-            gx = term.sh.coeff(gc)
-            gx = (gx if tomo is None else tomo.RT(gx)) * g
+            gx = term.sh.coeff(gc.mul_(g))   # scaled where the array is smallest
+            gx = gx if tomo is None else tomo.RT(gx)
         return (gx, gprb * g if ctx.needs_input_grad[1] else None, gpos * g if ctx.needs_input_grad[2] else None,
                 None, None, None, None)
 

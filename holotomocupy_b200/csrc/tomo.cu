@@ -986,7 +986,8 @@ extern "C" int ht_tomo_create(int n, int nz, int ntheta, const float* theta_host
   t->tw_n = twiddle_table(n, t->device);
   t->tw_2n = twiddle_table(2 * n, t->device);
   // two neighbouring angles' lines are at most n times their gap apart; up to
-  // three cells their windows share most of a box (see k_tgather)
+  // three cells their windows share most of a box (see k_tgather; 20 slices of 2048^2
+  // at 1800 angles, 3.6 cells apart at the rim: 3.3 ms one by one, 3.6 in pairs)
   int close = 0;
   for (int i = 0; i + 1 < ntheta; i += 2) close += (double)(ths[i + 1] - ths[i]) * n <= 3.0;
   t->pairs = 2 * close > ntheta / 2;
