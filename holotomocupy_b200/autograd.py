@@ -18,8 +18,12 @@ a complex output it is ``Re <grad_y, dy/dp>``):
 over angles is taken in complex128) into the BH data term
 (rec_mpi.py:517-813): ``F = 1/N sum (|D_k(prb_k exp(i S_k(coeff(R obj))))| - d)^2``
 over (angle, distance) images, optionally in angle chunks whose forward is
-recomputed in the backward pass (``torch.utils.checkpoint``), so that only one
-chunk's intermediates are held at a time.
+recomputed in the backward pass, so that only one chunk's intermediates are held
+at a time.  Where the fused cascade takes the inputs (``_use_fused``) a chunk is
+one function, ``ht_rec_forward`` and ``ht_rec_gradient`` in its backward pass
+(256^2 x 90 angles x 4 distances, value and gradients: 4.7 ms against 11.0
+operator by operator); else the operators are composed, with
+``torch.utils.checkpoint``.
 """
 import contextlib
 import ctypes

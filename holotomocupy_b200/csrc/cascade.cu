@@ -505,10 +505,8 @@ k_casc_resid512(float2* __restrict__ tmp, float2* __restrict__ x0c, const float*
   r512_dct2_tail(v, sm, t, tw4, tmp + row * N, valid);
 }
 
-// (five blocks an SM: with six, 80 registers a thread spill 92 bytes; 2.08 ms against
-// 2.11 for 900 images)
 template <int NDIR>
-__global__ void __launch_bounds__(32 * kR512Lines, 5)
+__global__ void __launch_bounds__(32 * kR512Lines, 6)
 k_casc_hess_q512(const float2* __restrict__ tmp, const float2* __restrict__ x0c, const float* __restrict__ data,
                  double* __restrict__ rows, CascDims D, const float2* __restrict__ tw4) {
   constexpr int N = kR512;
