@@ -86,7 +86,7 @@ class Shift:
         _lib.require_cuda(psi, "psi")
         real = self.obj_dtype == "float32"
         if real:   # the filter is real: the real part of its output is the filtered real part
-            x = (psi.real if psi.is_complex() else psi).to(torch.float32).contiguous()
+            x = (psi.real if psi.is_complex() else psi).to(torch.float32).contiguous().resolve_neg()
         else:
             x = psi.to(torch.complex64).contiguous()
         out = torch.empty_like(x)

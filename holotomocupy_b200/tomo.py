@@ -124,14 +124,24 @@ class Tomo:
                               _lib.ptr(sym) if sym is not None else None, float(scale), st)
         return res
 
-    @staticmethod
-    def _result(out, shape, dtype, device):
-        """(the array an operator writes, whether out still has to be copied from it)"""
-        if out is None:
-            return torch.empty(shape, dtype=dtype, device=device), False
-        if dtype.is_complex or (out.dtype == dtype and out.is_contiguous() and tuple(out.shape) == tuple(shape)):
-            return out, False
-        return torch.empty(shape, dtype=dtype, device=device), True
+    def _result(self, out, x, shape, nz):
+        """(the array the kernels write, whether out still has to be copied from
+        it) for an operator on the contiguous x of nz slices.  out itself is written where it
+        is an array of the result's type and layout on x's device; any other out
+        (on the host or another GPU, strided, of another type) is copied into, and
+        so is one that overlaps x when the volume takes several slabs, whose later
+        ones would read what the earlier ones wrote."""
+        if out is not None and not (out.is_conj() or out.is_neg()):
+            real, size = not x.is_complex(), math.prod(shape)
+            fits = (out.dtype == x.dtype and out.device == x.device and out.is_contiguous()
+                    and (tuple(out.shape) == shape and not out.requires_grad if real else out.numel() == size))
+            a, b, width = x.data_ptr(), out.data_ptr(), x.element_size()
+            apart = a + x.numel() * width <= b or b + size * width <= a
+            if fits and (apart or nz <= self._nz):
+                if not out.is_inference():
+                    torch.autograd.graph.increment_version(out)
+                return out, False
+        return torch.empty(shape, dtype=x.dtype, device=x.device), out is not None
 
     def R(self, obj, out=None):
         """Radon transform (tomo.py:56-86): [nz, n, n] -> [ntheta, nz, n] (any nz:
@@ -140,8 +150,8 @@ class Tomo:
         nz = obj.shape[0]
         if tuple(obj.shape[1:]) != (self.n, self.n):
             raise ValueError(f"obj must be [nz, {self.n}, {self.n}], got {tuple(obj.shape)}")
-        x = obj.to(torch.complex64 if obj.is_complex() else torch.float32).contiguous()
-        res, copy = self._result(out, (self.ntheta, nz, self.n), x.dtype, x.device)
+        x = obj.to(torch.complex64 if obj.is_complex() else torch.float32).contiguous().resolve_neg()
+        res, copy = self._result(out, x, (self.ntheta, nz, self.n), nz)
         self._R_into(x, res)
         return out.copy_(res) if copy else res
 
@@ -154,8 +164,8 @@ class Tomo:
         nz = data.shape[1]
         if data.shape[0] != self.ntheta or data.shape[2] != self.n:
             raise ValueError(f"data must be [{self.ntheta}, nz, {self.n}], got {tuple(data.shape)}")
-        x = data.to(torch.complex64 if data.is_complex() else torch.float32).contiguous()
-        res, copy = self._result(out, (nz, self.n, self.n), x.dtype, x.device)
+        x = data.to(torch.complex64 if data.is_complex() else torch.float32).contiguous().resolve_neg()
+        res, copy = self._result(out, x, (nz, self.n, self.n), nz)
         self._RT_into(x, res, scale=scale, sym=sym)
         return out.copy_(res) if copy else res
 

@@ -178,3 +178,53 @@ def test_R_RT_over_slice_batches(n, ntheta, nz):
     y = (rng.standard_normal((ntheta, nz, n)) + 1j * rng.standard_normal((ntheta, nz, n))).astype("complex64")
     assert rel_l2(t.R(torch.from_numpy(x).cuda()).cpu().numpy(), o.R(x)) < TOL
     assert rel_l2(t.RT(torch.from_numpy(y).cuda()).cpu().numpy(), o.RT(y)) < TOL
+
+
+@pytest.mark.parametrize("dtype", ["float32", "complex64"])
+@pytest.mark.parametrize("kind", ["host", "pinned", "strided", "wider type", "matching"])
+def test_R_RT_out_arrays(dtype, kind):
+    """out= on the host, strided, of a wider type or matching, by whole volumes
+    and by slabs: it holds the result when the call returns, and is returned; a
+    matching one is written in place and its version counts up."""
+    from holotomocupy_b200 import Tomo
+    n, nz, ntheta = 32, 6, 32
+    rng = np.random.default_rng(11)
+    theta = np.linspace(0, np.pi, ntheta, endpoint=False).astype("float32")
+    x, y = rng.standard_normal((nz, n, n)), rng.standard_normal((ntheta, nz, n))
+    if dtype == "complex64":
+        x, y = x + 1j * rng.standard_normal(x.shape), y + 1j * rng.standard_normal(y.shape)
+    x, y = (torch.from_numpy(a.astype(dtype)).cuda() for a in (x, y))
+    for t in (Tomo(n, nz, theta, 0.9), Tomo(n, 4, theta, 0.9)):
+        for op, a in ((t.R, x), (t.RT, y)):
+            ref = op(a)
+            out = {"host": lambda: torch.empty(ref.shape, dtype=ref.dtype),
+                   "pinned": lambda: torch.empty(ref.shape, dtype=ref.dtype, pin_memory=True),
+                   "strided": lambda: torch.empty(ref.shape + (2,), dtype=ref.dtype, device="cuda")[..., 1],
+                   "wider type": lambda: torch.empty(ref.shape, dtype=torch.promote_types(ref.dtype, torch.float64),
+                                                     device="cuda"),
+                   "matching": lambda: torch.empty_like(ref)}[kind]()
+            version = out._version
+            assert op(a, out=out) is out and out._version > version
+            assert torch.equal(out.to(ref.device, ref.dtype), ref)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "complex64"])
+@pytest.mark.parametrize("capacity", [10, 24])
+def test_R_RT_out_over_the_input(dtype, capacity):
+    """out= the input itself, or an array that starts inside it, in one slab and
+    in three: the result of a separate out."""
+    from holotomocupy_b200 import Tomo
+    n = 24   # as many angles and slices as cells: R and R^T keep the shape
+    rng = np.random.default_rng(12)
+    t = Tomo(n, capacity, np.linspace(0, np.pi, n, endpoint=False).astype("float32"), 0.9)
+    x = rng.standard_normal((n, n, n))
+    if dtype == "complex64":
+        x = x + 1j * rng.standard_normal(x.shape)
+    x = torch.from_numpy(x.astype(dtype)).cuda()
+    for op in (t.R, t.RT):
+        y = x.clone()
+        ref = op(x)
+        assert torch.equal(op(y, out=y), ref)
+        big = torch.cat([x.reshape(-1), x.reshape(-1)[:5]])
+        view = big[5:].view(n, n, n)
+        assert torch.equal(op(big[:n ** 3].view(n, n, n), out=view), ref)
