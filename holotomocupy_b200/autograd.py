@@ -227,15 +227,22 @@ class DataFidelity(torch.nn.Module):
         up to twice their width (its rows' shared memory), contiguous arrays
         of the operators' types on their device, and gives no gradient for the
         data or the magnifications; a handle is not made while a graph is being
-        captured.  Anything else goes operator by operator."""
-        odt = torch.complex64 if self.sh.obj_dtype == "complex64" else torch.float32
+        captured.  It stands for the operators as they were made: a propagator set
+        to the padded grid (``_use_cufftdx``) and operators of other sizes or types
+        put in the place of the first ones go operator by operator, like the rest."""
+        sh, prop = self.sh, self.prop
+        if type(sh) is not Shift or type(prop) is not Propagation:
+            return False
+        odt = torch.complex64 if sh.obj_dtype == "complex64" else torch.float32
         shape = (self.ntheta, self.nzobj, self.nobj) if proj else (self.nzobj, self.nobj, self.nobj)
         nd, f32 = (self.ndist, self.nz, self.n), torch.float32
         want = ((x, odt, shape), (prb, torch.complex64, nd), (pos, f32, (self.ntheta, self.ndist, 2)),
                 (mag, f32, (self.ntheta, self.ndist)), (data, f32, (self.ntheta,) + nd))
         return (self.n in self.FUSED_ROWS and self.nobj <= 2 * self.n and not data.requires_grad
+                and prop._use_cufftdx and (prop.ndist, prop.nz, prop.n) == nd and prop.device == sh.device
+                and (sh.n, sh.nz, sh.npsi, sh.nzpsi) == (self.n, self.nz, self.nobj, self.nzobj)
                 and all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.dtype == dt and tuple(t.shape) == sz
-                        and t.device == self.sh.device and t.is_contiguous() and not t.is_conj() and not t.is_neg()
+                        and t.device == sh.device and t.is_contiguous() and not t.is_conj() and not t.is_neg()
                         for t, dt, sz in want)
                 and not torch.cuda.is_current_stream_capturing())
 

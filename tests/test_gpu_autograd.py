@@ -226,3 +226,43 @@ def test_fidelity_fused_equals_operator_by_operator(n, nobj, obj_dtype, chunk, p
         assert a.dtype == b.dtype and a.shape == b.shape
         assert torch.isfinite(torch.view_as_real(a) if a.is_complex() else a).all()
         assert rel_l2(a.cpu().numpy(), b.cpu().numpy()) < 1e-5, rel_l2(a.cpu().numpy(), b.cpu().numpy())
+
+
+def _small_fidelity(seed=5, n=32, ntheta=5, ndist=2, chunk=None, obj_dtype="complex64"):
+    """A data term the fused cascade takes, and its inputs (obj, prb, pos, mag, data)."""
+    from holotomocupy_b200.autograd import DataFidelity
+    rng = np.random.default_rng(seed)
+    theta = np.linspace(0, np.pi, ntheta, endpoint=False).astype("float32")
+    fid = DataFidelity.create(n, n, n, n, theta, ndist, 7.3e-11, 20e-9, np.linspace(3e-3, 5e-3, ndist), 0.9, chunk,
+                              obj_dtype)
+    obj = (0.05 * rng.standard_normal((n, n, n))).astype(obj_dtype)
+    prb = (1 + 0.1 * rng.standard_normal((ndist, n, n)) + 0.1j).astype("complex64")
+    pos = rng.uniform(-3, 3, (ntheta, ndist, 2)).astype("float32")
+    mag = rng.uniform(0.9, 1.0, (ntheta, ndist)).astype("float32")
+    data = (1 + 0.1 * rng.standard_normal((ntheta, ndist, n, n))).astype("float32")
+    return fid, [cuda(a) for a in (obj, prb, pos, mag, data)]
+
+
+def test_fidelity_follows_its_operators_settings():
+    """The propagator set to the padded grid, or one of another size or of a type
+    of its own in its place: operator by operator, as the operators themselves go."""
+    from holotomocupy_b200 import Propagation
+
+    class Half(Propagation):
+        def D(self, psi, j):
+            return 0.5 * super().D(psi, j)
+    fid, args = _small_fidelity()
+    ref = fid(*args)
+    calls = []
+    padded = fid.prop._padded
+    fid.prop._padded = lambda *a: calls.append(a[1]) or padded(*a)
+    fid.prop._use_cufftdx = False
+    assert not fid._use_fused(*args, False)
+    assert rel_l2(fid(*args).cpu().numpy(), ref.cpu().numpy()) < 1e-5
+    assert calls == [0, 1]
+    fid.prop = Propagation(32, 32, 5, 3, 7.3e-11, 20e-9, [3e-3, 5e-3, 9e-3])
+    assert not fid._use_fused(*args, False)
+    assert rel_l2(fid(*args).cpu().numpy(), ref.cpu().numpy()) < 1e-5
+    fid.prop = Half(32, 32, 5, 2, 7.3e-11, 20e-9, [3e-3, 5e-3])
+    assert not fid._use_fused(*args, False)
+    assert abs(fid(*args) - 0.25) < 0.05   # amplitudes near 1/2 under data near 1
