@@ -71,6 +71,10 @@ SIGNATURES = {
     "ht_ktimer_arm": [ctypes.c_char_p, _c_int],
     "ht_ktimer_read": [ctypes.c_char_p, ctypes.POINTER(_c_double), ctypes.POINTER(_c_long), ctypes.POINTER(_c_double)],
     "ht_rec_create": [_c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _vp, ctypes.POINTER(_vp)],
+    "ht_rec_workspace_bytes": [_c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _vp, _c_int,
+                               ctypes.POINTER(ctypes.c_size_t)],
+    "ht_rec_create_in": [_c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _vp, _c_int, _vp, ctypes.c_size_t,
+                         ctypes.POINTER(_vp)],
     "ht_rec_destroy": [_vp],
     "ht_rec_forward": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
     "ht_rec_gradient": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _c_float, _c_float, _c_int, _vp],

@@ -27,7 +27,6 @@ operator by operator); else the operators are composed, with
 """
 import contextlib
 import ctypes
-import threading
 
 import numpy as np
 import torch
@@ -98,73 +97,72 @@ class _ProbeMul(torch.autograd.Function):
         return gprb, gx
 
 
+class _Cascade:
+    """The fused cascade of one angle chunk, over the operators that the data term
+    has at the time of the call: F and the gradients come from handles that live
+    for a call, in workspaces of torch's allocator."""
+
+    def __init__(self, term, ntheta, tomo):
+        self.sh, self.prop, self.tomo = term.sh, term.prop, tomo
+        self.data_size = term.data_size
+        self.sizes = (term.n, term.nz, term.nobj, term.nzobj, ntheta, term.ndist,
+                      int(term.sh.obj_dtype == "complex64"))
+
+    def coeff(self, x):
+        return self.sh.coeff(x if self.tomo is None else self.tomo.R(x.contiguous()))
+
+    @contextlib.contextmanager
+    def handle(self, forward_only=False):
+        with torch.cuda.device(self.sh.device):
+            size, h = ctypes.c_size_t(), ctypes.c_void_p()
+            args = (*self.sizes, self.prop._h, int(forward_only))
+            _lib.call("ht_rec_workspace_bytes", *args, ctypes.byref(size))
+            work = torch.empty(size.value, dtype=torch.uint8, device=self.sh.device)
+            _lib.call("ht_rec_create_in", *args, _lib.ptr(work), size.value, ctypes.byref(h))
+            try:
+                _lib.call("ht_rec_set_data_size", h, float(self.data_size))
+                _lib.call("ht_rec_set_zero_gradient", h, 1)   # torch.abs has gradient 0 at 0
+                yield h
+            finally:
+                _lib.lib().ht_rec_destroy(h)
+
+
 class _ChunkMisfit(torch.autograd.Function):
     """1/N sum (|D_k(prb_k exp(i S_k(coeff(x))))| - d)^2 of one angle chunk by the
     fused cascade (ht_rec_forward; ht_rec_gradient in the backward pass, which
     repeats the forward from the saved inputs, so that no image stack is held
-    between the two).  x is the chunk's projections, or with tomo the object."""
+    between the two).  x is the chunk's projections, or the object where the
+    cascade has a Radon transform."""
 
     @staticmethod
-    def forward(ctx, x, prb, pos, mag, data, term, tomo):
-        ctx.term, ctx.tomo = term, tomo
+    def forward(ctx, x, prb, pos, mag, data, cascade):
+        ctx.cascade = cascade
         ctx.save_for_backward(x, prb, pos, mag, data)
-        c = term.sh.coeff(x if tomo is None else tomo.R(x.contiguous()))
+        c = cascade.coeff(x)
         f = torch.empty(1, dtype=torch.float64, device=x.device)
-        with term.handle(len(pos)) as h:
+        with cascade.handle(forward_only=True) as h:
             _lib.call("ht_rec_forward", h, _lib.ptr(c), _lib.ptr(pos), _lib.ptr(mag), _lib.ptr(prb), _lib.ptr(data),
                       None, _lib.ptr(f), _lib.stream_ptr())
-        return (f[0] / term.data_size).to(torch.float32)
+        return (f[0] / cascade.data_size).to(torch.float32)
 
     @staticmethod
     def backward(ctx, g):
         x, prb, pos, mag, data = ctx.saved_tensors
-        term, tomo = ctx.term, ctx.tomo
-        c = term.sh.coeff(x if tomo is None else tomo.R(x.contiguous()))
+        cascade = ctx.cascade
+        c = cascade.coeff(x)
         gc, gpos, gprb = torch.empty_like(c), torch.empty_like(pos), torch.empty_like(prb)
-        with term.handle(len(pos)) as h:
+        with cascade.handle() as h:
             _lib.call("ht_rec_gradient", h, _lib.ptr(c), _lib.ptr(pos), _lib.ptr(mag), _lib.ptr(prb),
                       _lib.ptr(data), _lib.ptr(gc), _lib.ptr(gpos), _lib.ptr(gprb), None, 1.0, 1.0, 0,
                       _lib.stream_ptr())
+        del c
         gx = None
         if ctx.needs_input_grad[0]:
-            gx = term.sh.coeff(gc.mul_(g))   # scaled where the array is smallest
-            gx = gx if tomo is None else tomo.RT(gx)
+            gx = cascade.sh.coeff(gc.mul_(g))   # scaled where the array is smallest
+            del gc
+            gx = gx if cascade.tomo is None else cascade.tomo.RT(gx)
         return (gx, gprb * g if ctx.needs_input_grad[1] else None, gpos * g if ctx.needs_input_grad[2] else None,
-                None, None, None, None)
-
-
-class _Handles:
-    """Fused-cascade handles of one DataFidelity, by (angles, stream): a handle's
-    workspace serves one call at a time, and calls on one stream run in order.
-    The four last used are kept."""
-
-    KEEP = 4
-
-    def __init__(self):
-        self.lock = threading.Lock()
-        self.items = {}
-
-    def take(self, key, make):
-        with self.lock:
-            h = self.items.pop(key, None)
-        return h if h is not None else make()
-
-    def put(self, key, h):
-        with self.lock:
-            old = self.items.pop(key, None)
-            self.items[key] = h
-            extra = [] if old is None else [old]
-            while len(self.items) > self.KEEP:
-                extra.append(self.items.pop(next(iter(self.items))))
-        for e in extra:
-            _lib.lib().ht_rec_destroy(e)
-
-    def __del__(self):
-        for h in self.items.values():
-            try:
-                _lib.lib().ht_rec_destroy(h)
-            except Exception:
-                pass
+                None, None, None)
 
 
 def radon(obj, tomo):
@@ -189,7 +187,8 @@ class DataFidelity(torch.nn.Module):
     ``theta``, ``ndist`` distances (metres), probe [ndist, nz, n], positions
     [ntheta, ndist, 2] (y, x) and magnifications [ntheta, ndist].  With
     ``chunk`` the angles are processed ``chunk`` at a time and each chunk's
-    forward is recomputed during the backward pass."""
+    forward is recomputed during the backward pass.  Its Radon transforms own one
+    workspace each, so one DataFidelity serves one stream at a time."""
 
     FUSED_ROWS = (32, 64, 128, 256, 384, 512, 768, 1024, 2048)   # detector row lengths of the fused cascade
 
@@ -204,7 +203,6 @@ class DataFidelity(torch.nn.Module):
         self.bounds = [(a, min(a + self.chunk, self.ntheta)) for a in range(0, self.ntheta, self.chunk)]
         self.tomos = [Tomo(nobj, nzobj, theta[a:b], mask_r, norm_ntheta=self.ntheta) for a, b in self.bounds]
         self.sh, self.prop = sh, prop
-        self._handles = _Handles()
 
     @classmethod
     def create(cls, n, nz, nobj, nzobj, theta, ndist, wavelength, voxelsize, distance, mask_r=None, chunk=None,
@@ -225,11 +223,12 @@ class DataFidelity(torch.nn.Module):
     def _use_fused(self, x, prb, pos, mag, data, proj):
         """The fused cascade takes detectors of its row lengths under objects of
         up to twice their width (its rows' shared memory), contiguous arrays
-        of the operators' types on their device, and gives no gradient for the
-        data or the magnifications; a handle is not made while a graph is being
-        captured.  It stands for the operators as they were made: a propagator set
-        to the padded grid (``_use_cufftdx``) and operators of other sizes or types
-        put in the place of the first ones go operator by operator, like the rest."""
+        of the operators' types on their device, a normalisation of at least the
+        number of samples, and gives no gradient for the data or the
+        magnifications.  It stands for the operators as they were made: a
+        propagator set to the padded grid (``_use_cufftdx``) and operators of other
+        sizes or types put in the place of the first ones go operator by operator,
+        like the rest."""
         sh, prop = self.sh, self.prop
         if type(sh) is not Shift or type(prop) is not Propagation:
             return False
@@ -244,26 +243,7 @@ class DataFidelity(torch.nn.Module):
                 and all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.dtype == dt and tuple(t.shape) == sz
                         and t.device == sh.device and t.is_contiguous() and not t.is_conj() and not t.is_neg()
                         for t, dt, sz in want)
-                and not torch.cuda.is_current_stream_capturing())
-
-    def _make_handle(self, ntheta):
-        h = ctypes.c_void_p()
-        _lib.call("ht_rec_create", self.n, self.nz, self.nobj, self.nzobj, ntheta, self.ndist,
-                  int(self.sh.obj_dtype == "complex64"), self.prop._h, ctypes.byref(h))
-        _lib.call("ht_rec_set_data_size", h, float(self.data_size))
-        _lib.call("ht_rec_set_zero_gradient", h, 1)   # torch.abs has gradient 0 at 0
-        return h
-
-    @contextlib.contextmanager
-    def handle(self, ntheta):
-        """A cascade handle for ntheta angles on the current stream."""
-        key = (ntheta, torch.cuda.current_stream(self.sh.device).cuda_stream)
-        with torch.cuda.device(self.sh.device):
-            h = self._handles.take(key, lambda: self._make_handle(ntheta))
-            try:
-                yield h
-            finally:
-                self._handles.put(key, h)
+                and self.data_size >= self.ntheta * self.ndist * self.nz * self.n)
 
     def _term(self, proj, prb, pos, mag, data):
         out = proj.new_zeros((), dtype=torch.float32).real
@@ -283,8 +263,8 @@ class DataFidelity(torch.nn.Module):
         total = None
         if self._use_fused(x, prb, pos, mag, data, proj):
             for i, (a, b) in enumerate(self.bounds):
-                f = _ChunkMisfit.apply(x[a:b] if proj else x, prb, pos[a:b], mag[a:b], data[a:b], self,
-                                       None if proj else self.tomos[i])
+                f = _ChunkMisfit.apply(x[a:b] if proj else x, prb, pos[a:b], mag[a:b], data[a:b],
+                                       _Cascade(self, b - a, None if proj else self.tomos[i]))
                 total = f if total is None else total + f
             return total
         for i, (a, b) in enumerate(self.bounds):

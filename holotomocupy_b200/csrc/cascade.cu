@@ -34,6 +34,7 @@
 #include <algorithm>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 namespace ht {
@@ -1195,9 +1196,11 @@ struct ht_rec_s {
   ht::CascDims D;
   int ntheta, is_complex, device;
   const ht_prop_s* prop;
-  float2* x0;      // [nimg, nz, n]
-  float2* P;       // [nimg, nz, n]
-  float2* tmp;     // [2, nimg, nz, n]
+  void* owned;     // the workspace, if the handle allocated it
+  int forward_only;
+  float2* x0;      // [nimg, nz, n]; null in a handle for the forward pass
+  float2* P;       // [nimg, nz, n]; null likewise
+  float2* tmp;     // [2, nimg, nz, n]; one spectrum for the forward pass
   double* acc_img; // [nimg, kNAcc]
   double* glob;    // [kNGlob]
   double* rows;    // [nimg * nz, kRowKMax] per-row sums of the row kernels
@@ -1205,65 +1208,104 @@ struct ht_rec_s {
   double ndata;    // N of the objective's 2/N: ntheta*ndist*nz*n, or the whole problem's for an angle chunk
 };
 
-extern "C" int ht_rec_create(int n, int nz, int nobj, int nzobj, int ntheta, int ndist, int is_complex,
-                             ht_prop_s* prop, ht_rec_s** out) {
-  using namespace ht;
-  HT_REQUIRE(out && prop, "ht_rec_create: null pointer");
-  HT_REQUIRE(n > 0 && nz > 0 && nobj > 0 && nzobj > 0 && ntheta > 0 && ndist > 0, "ht_rec_create: bad sizes");
+namespace ht {
+// The handle's arrays in one workspace, each at a multiple of 512 bytes; the
+// bytes it takes.  base may be null (sizes only).
+static size_t rec_layout(ht_rec_s* r, char* base) {
+  const size_t nimg = (size_t)r->D.nimg, img = nimg * r->D.nz * r->D.n;
+  size_t at = 0;
+  auto take = [&](auto& p, size_t count) {
+    p = base && count ? reinterpret_cast<std::decay_t<decltype(p)>>(base + at) : nullptr;
+    at += (count * sizeof(*p) + 511) / 512 * 512;
+  };
+  take(r->x0, r->forward_only ? 0 : img);
+  take(r->P, r->forward_only ? 0 : img);
+  // tmp: two spectra for the Hessian pass; during the gradient pass its
+  // second part holds the horizontal S^T rows [nimg, nz, nobj] of T
+  const size_t hrow = (nimg * r->D.nz * r->D.nobj * (r->is_complex ? 8 : 4) + 7) / 8;
+  take(r->tmp, r->forward_only ? img : img + std::max(img, hrow));
+  take(r->acc_img, nimg * kNAcc);
+  take(r->glob, kNGlob);
+  take(r->rows, nimg * r->D.nz * kRowKMax);
+  take(r->imgs, nimg * kRowKMax);
+  return at;
+}
+
+// Size checks of a handle, and the handle without its workspace.
+static int rec_new(const char* name, int n, int nz, int nobj, int nzobj, int ntheta, int ndist, int is_complex,
+                   ht_prop_s* prop, int forward_only, ht_rec_s* r) {
+  HT_REQUIRE(prop, std::string(name) + ": null pointer");
+  HT_REQUIRE(n > 0 && nz > 0 && nobj > 0 && nzobj > 0 && ntheta > 0 && ndist > 0, std::string(name) + ": bad sizes");
   int pn, pnz, pnd;
   prop_dims(prop, &pn, &pnz, &pnd);
-  HT_REQUIRE(pn == n && pnz == nz && pnd == ndist, "ht_rec_create: propagator sizes differ");
+  HT_REQUIRE(pn == n && pnz == nz && pnd == ndist, std::string(name) + ": propagator sizes differ");
   bool n_ok = false;
 #define X(S) n_ok = n_ok || (n == S);
   HT_REC_SIZES(X)
 #undef X
   if (!n_ok) {
-    set_error("ht_rec_create: n must be one of 32, 64, 128, 256, 384, 512, 768, 1024, 2048");
+    set_error(std::string(name) + ": n must be one of 32, 64, 128, 256, 384, 512, 768, 1024, 2048");
     return kUnsupported;
   }
-  ht_rec_s* r = new ht_rec_s{};
+  *r = ht_rec_s{};
   r->D = CascDims{n, nz, nobj, nzobj, ndist, (long)ntheta * ndist};
   r->ntheta = ntheta;
   r->ndata = (double)ntheta * ndist * nz * n;
   r->is_complex = is_complex ? 1 : 0;
+  r->forward_only = forward_only ? 1 : 0;
   r->prop = prop;
   cudaGetDevice(&r->device);
-  const size_t img = (size_t)ntheta * ndist * nz * n;
-  cudaError_t e = cudaMalloc(&r->x0, sizeof(float2) * img);
-  if (e == cudaSuccess) e = cudaMalloc(&r->P, sizeof(float2) * img);
-  // tmp: two spectra for the Hessian pass; during the gradient pass its
-  // second part holds the horizontal S^T rows [nimg, nz, nobj] of T
-  const size_t hrow = ((size_t)ntheta * ndist * nz * nobj * (is_complex ? 8 : 4) + 7) / 8;
-  if (e == cudaSuccess) e = cudaMalloc(&r->tmp, sizeof(float2) * (img + std::max(img, hrow)));
-  if (e == cudaSuccess) e = cudaMalloc(&r->acc_img, sizeof(double) * (size_t)ntheta * ndist * kNAcc);
-  if (e == cudaSuccess) e = cudaMalloc(&r->glob, sizeof(double) * kNGlob);
-  if (e == cudaSuccess) e = cudaMalloc(&r->rows, sizeof(double) * (size_t)ntheta * ndist * nz * kRowKMax);
-  if (e == cudaSuccess) e = cudaMalloc(&r->imgs, sizeof(double) * (size_t)ntheta * ndist * kRowKMax);
+  return kOk;
+}
+}  // namespace ht
+
+extern "C" int ht_rec_create(int n, int nz, int nobj, int nzobj, int ntheta, int ndist, int is_complex,
+                             ht_prop_s* prop, ht_rec_s** out) {
+  using namespace ht;
+  HT_REQUIRE(out, "ht_rec_create: null pointer");
+  ht_rec_s r;
+  const int st = rec_new("ht_rec_create", n, nz, nobj, nzobj, ntheta, ndist, is_complex, prop, 0, &r);
+  if (st != kOk) return st;
+  void* base = nullptr;
+  const cudaError_t e = cudaMalloc(&base, rec_layout(&r, nullptr));
   if (e != cudaSuccess) {
     set_error(std::string("ht_rec_create: ") + cudaGetErrorString(e));
-    cudaFree(r->x0);
-    cudaFree(r->P);
-    cudaFree(r->tmp);
-    cudaFree(r->acc_img);
-    cudaFree(r->glob);
-    cudaFree(r->rows);
-    cudaFree(r->imgs);
-    delete r;
     return kCudaError;
   }
-  *out = r;
+  r.owned = base;
+  rec_layout(&r, static_cast<char*>(base));
+  *out = new ht_rec_s(r);
+  return kOk;
+}
+
+extern "C" int ht_rec_workspace_bytes(int n, int nz, int nobj, int nzobj, int ntheta, int ndist, int is_complex,
+                                      ht_prop_s* prop, int forward_only, size_t* bytes) {
+  using namespace ht;
+  HT_REQUIRE(bytes, "ht_rec_workspace_bytes: null pointer");
+  ht_rec_s r;
+  const int st =
+      rec_new("ht_rec_workspace_bytes", n, nz, nobj, nzobj, ntheta, ndist, is_complex, prop, forward_only, &r);
+  if (st != kOk) return st;
+  *bytes = rec_layout(&r, nullptr);
+  return kOk;
+}
+
+extern "C" int ht_rec_create_in(int n, int nz, int nobj, int nzobj, int ntheta, int ndist, int is_complex,
+                                ht_prop_s* prop, int forward_only, void* workspace, size_t bytes, ht_rec_s** out) {
+  using namespace ht;
+  HT_REQUIRE(out && workspace, "ht_rec_create_in: null pointer");
+  ht_rec_s r;
+  const int st = rec_new("ht_rec_create_in", n, nz, nobj, nzobj, ntheta, ndist, is_complex, prop, forward_only, &r);
+  if (st != kOk) return st;
+  HT_REQUIRE(reinterpret_cast<size_t>(workspace) % 512 == 0, "ht_rec_create_in: workspace must be 512-byte aligned");
+  HT_REQUIRE(rec_layout(&r, static_cast<char*>(workspace)) <= bytes, "ht_rec_create_in: workspace too small");
+  *out = new ht_rec_s(r);
   return kOk;
 }
 
 extern "C" int ht_rec_destroy(ht_rec_s* r) {
   if (!r) return ht::kOk;
-  cudaFree(r->x0);
-  cudaFree(r->P);
-  cudaFree(r->tmp);
-  cudaFree(r->acc_img);
-  cudaFree(r->glob);
-  cudaFree(r->rows);
-  cudaFree(r->imgs);
+  if (r->owned) cudaFree(r->owned);  // not called at all for the caller's memory: it would end a graph capture
   delete r;
   return ht::kOk;
 }
@@ -1505,6 +1547,7 @@ extern "C" int ht_rec_gradient(ht_rec_s* r, const void* c, const float* pos, con
                                float scale_prb, int accumulate, void* stream) {
   using namespace ht;
   HT_REQUIRE(r && c && pos && mag && prb && data && gc && gpos && gprb, "ht_rec_gradient: null pointer");
+  HT_REQUIRE(!r->forward_only, "ht_rec_gradient: the handle is for the forward pass");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   HT_CHECK_CUDA(cudaMemsetAsync(r->glob, 0, sizeof(double) * kNGlob, st));
   HT_CHECK_CUDA(cudaMemsetAsync(r->acc_img, 0, sizeof(double) * r->D.nimg * kNAcc, st));
@@ -1541,6 +1584,7 @@ extern "C" int ht_rec_hessian(ht_rec_s* r, const void* c, const float* pos, cons
                               void* stream) {
   using namespace ht;
   HT_REQUIRE(r && c && pos && mag && prb && data && cy && posy && prby && out, "ht_rec_hessian: null pointer");
+  HT_REQUIRE(!r->forward_only, "ht_rec_hessian: the handle is for the forward pass");
   HT_REQUIRE(ndir == 1 || (ndir == 2 && cz && posz && prbz), "ht_rec_hessian: ndir must be 1, or 2 with z given");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // clear the Hessian slots only: the gradient pass's per-image terms stay

@@ -17,6 +17,8 @@
 #ifndef HOLOTOMO_B200_H
 #define HOLOTOMO_B200_H
 
+#include <stddef.h>
+
 #ifdef __cplusplus
 extern "C" {
 #endif
@@ -217,14 +219,23 @@ int ht_shift_dSadj(ht_shift_s* s, const void* c, const float* r, const float* ma
  * coefficients of proj (complex64, or float32 when is_complex = 0);
  * pos [ntheta, ndist, 2] float32 (y, x); mag [ntheta, ndist] float32;
  * prb [ndist, nz, n] complex64; data [ntheta, ndist, nz, n] float32
- * amplitudes.  The handle owns 4*nimg*nz*n complex64 samples of workspace:
- * caches of the last gradient call that ht_rec_hessian reads, so call
- * ht_rec_gradient first with the same state.
+ * amplitudes.  A handle works in 4*nimg*nz*n complex64 samples of workspace
+ * (more where nobj > n), its own or the caller's: caches of the last gradient
+ * call that ht_rec_hessian reads, so call ht_rec_gradient first with the same
+ * state.
  * --------------------------------------------------------------------- */
 typedef struct ht_rec_s ht_rec_s;
 
 int ht_rec_create(int n, int nz, int nobj, int nzobj, int ntheta, int ndist, int is_complex, ht_prop_s* prop,
                   ht_rec_s** out);
+/* A handle in the caller's device memory (512-byte aligned, of at least
+ * ht_rec_workspace_bytes bytes, kept until the handle's last call has run).  Makes
+ * no device allocation and no synchronisation.  forward_only = 1: for
+ * ht_rec_forward alone, in about a quarter of the memory. */
+int ht_rec_workspace_bytes(int n, int nz, int nobj, int nzobj, int ntheta, int ndist, int is_complex, ht_prop_s* prop,
+                           int forward_only, size_t* bytes);
+int ht_rec_create_in(int n, int nz, int nobj, int nzobj, int ntheta, int ndist, int is_complex, ht_prop_s* prop,
+                     int forward_only, void* workspace, size_t bytes, ht_rec_s** out);
 int ht_rec_destroy(ht_rec_s* r);
 
 /* Forward model.  With amp != NULL: amp[ntheta, ndist, nz, n] = |x0|

@@ -266,3 +266,126 @@ def test_fidelity_follows_its_operators_settings():
     fid.prop = Half(32, 32, 5, 2, 7.3e-11, 20e-9, [3e-3, 5e-3])
     assert not fid._use_fused(*args, False)
     assert abs(fid(*args) - 0.25) < 0.05   # amplitudes near 1/2 under data near 1
+
+
+def _value_and_grads(fid, args, proj=False):
+    t = [a.clone().requires_grad_() for a in args[:3]]
+    f = fid(*t, *args[3:], proj=proj)
+    return [f.detach()] + list(torch.autograd.grad(f, t))
+
+
+def test_fidelity_takes_a_replaced_propagator():
+    """A propagator put in the place of the first one is the one that counts, also
+    after the first is gone and its tables' memory is in other hands, and a
+    backward pass keeps the operators its forward pass had."""
+    from holotomocupy_b200 import Propagation
+    fid, args = _small_fidelity()
+    first = _value_and_grads(fid, args)
+    t = [a.clone().requires_grad_() for a in args[:3]]
+    f = fid(*t, *args[3:])
+    fid.prop = Propagation(32, 32, 5, 2, 7.3e-11, 20e-9, [9e-3, 12e-3])
+    got = _value_and_grads(fid, args)
+    other, _ = _small_fidelity()
+    other.prop = fid.prop
+    other._use_fused = lambda *a: False
+    for a, b in zip(got, _value_and_grads(other, args)):
+        assert rel_l2(a.cpu().numpy(), b.cpu().numpy()) < 1e-5
+    assert abs(got[0] - first[0]) > 1e-3 * first[0]
+    for a, b in zip(torch.autograd.grad(f, t), first[1:]):
+        assert torch.equal(a, b)
+
+
+def test_fidelity_holds_no_memory_between_calls():
+    """The cascade's workspaces come from torch's allocator and go back with the
+    call, ragged chunks and several streams included: after a call nothing is
+    held, inside torch or outside."""
+    fid, args = _small_fidelity(n=64, ntheta=7, chunk=4)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    for stream in (torch.cuda.current_stream(), torch.cuda.Stream(), torch.cuda.Stream()):
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            _value_and_grads(fid, args)
+        torch.cuda.synchronize()
+    held, free = torch.cuda.memory_allocated(), torch.cuda.mem_get_info()[0] + torch.cuda.memory_reserved()
+    for stream in (torch.cuda.current_stream(), torch.cuda.Stream(), torch.cuda.Stream()):
+        with torch.cuda.stream(stream):
+            _value_and_grads(fid, args)
+        torch.cuda.synchronize()
+    assert torch.cuda.memory_allocated() == held
+    assert torch.cuda.mem_get_info()[0] + torch.cuda.memory_reserved() == free
+
+
+@pytest.mark.parametrize("n,ntheta,ndist,chunk", [(64, 45, 2, None), (64, 46, 4, 23)])
+def test_fidelity_peak_memory_is_that_of_the_operators(n, ntheta, ndist, chunk):
+    """Peak of a value, and of a value with gradients, over the inputs: the fused
+    cascade's at most that of the composition and a tenth."""
+    peaks = {}
+    for fused in (True, False):
+        fid, args = _small_fidelity(n=n, ntheta=ntheta, ndist=ndist, chunk=chunk)
+        if not fused:
+            fid._use_fused = lambda *a: False
+        for grads in (False, True):
+            run = (lambda: _value_and_grads(fid, args)) if grads else (lambda: fid(*args))
+            run()
+            torch.cuda.synchronize()
+            torch.cuda.reset_peak_memory_stats()
+            base = torch.cuda.memory_allocated()
+            run()
+            peaks[fused, grads] = torch.cuda.max_memory_allocated() - base
+    assert peaks[True, False] <= 1.1 * peaks[False, False], peaks
+    assert peaks[True, True] <= 1.1 * peaks[False, True], peaks
+
+
+def test_fidelity_under_capture():
+    """Value and gradients recorded into a graph and replayed on other inputs."""
+    fid, args = _small_fidelity(chunk=3)
+    _, other = _small_fidelity(seed=6, chunk=3)
+    ref = _value_and_grads(fid, other)
+    bufs = [a.clone() for a in args]
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        _value_and_grads(fid, bufs)
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = _value_and_grads(fid, bufs)
+    for b, o in zip(bufs, other):
+        b.copy_(o)
+    graph.replay()
+    torch.cuda.synchronize()
+    for a, b in zip(got, ref):
+        assert torch.equal(a, b)
+
+
+def test_fidelity_from_two_threads():
+    """Two data terms of one shift and one propagator, each in a thread and on a
+    stream of its own: the values and gradients of one after the other."""
+    import threading
+
+    from holotomocupy_b200.autograd import DataFidelity
+    fid, args = _small_fidelity(n=64, ntheta=6, chunk=4)
+    fids = [fid, DataFidelity(fid.sh, fid.prop, np.linspace(0, np.pi, 6, endpoint=False), 0.9, 64, 64, 4)]
+    sets = [args, _small_fidelity(seed=8, n=64, ntheta=6, chunk=4)[1]]
+    refs = [_value_and_grads(f, a) for f, a in zip(fids, sets)]
+    torch.cuda.synchronize()
+    res, errors = [None, None], []
+
+    def work(i):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(20):
+                    res[i] = _value_and_grads(fids[i], sets[i])
+                torch.cuda.current_stream().synchronize()
+        except Exception as e:   # shown by the assertion below
+            errors.append(e)
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for got, ref in zip(res, refs):
+        for a, b in zip(got, ref):
+            assert torch.equal(a, b)
