@@ -24,12 +24,17 @@ one function, ``ht_rec_forward`` and ``ht_rec_gradient`` in its backward pass
 (256^2 x 90 angles x 4 distances, value and gradients: 4.7 ms against 11.0
 operator by operator); else the operators are composed, with
 ``torch.utils.checkpoint``.
+
+The backward passes are library calls, which autograd does not see into: the
+operators and the data term are differentiable once, and a derivative of their
+gradients is refused.
 """
 import contextlib
 import ctypes
 
 import numpy as np
 import torch
+from torch.autograd.function import once_differentiable
 from torch.utils.checkpoint import checkpoint
 
 from . import _lib
@@ -45,6 +50,7 @@ class _Radon(torch.autograd.Function):
         return tomo.R(obj.contiguous())
 
     @staticmethod
+    @once_differentiable
     def backward(ctx, g):
         return ctx.tomo.RT(g.contiguous()), None
 
@@ -58,6 +64,7 @@ class _Shift(torch.autograd.Function):
         return sh.S(c, pos, mag)
 
     @staticmethod
+    @once_differentiable
     def backward(ctx, g):
         c, pos, mag = ctx.saved_tensors
         sh = ctx.sh
@@ -73,6 +80,7 @@ class _Propagate(torch.autograd.Function):
         return prop.D(psi.contiguous(), j)
 
     @staticmethod
+    @once_differentiable
     def backward(ctx, g):
         return ctx.prop.DT(g.contiguous(), ctx.j), None, None
 
@@ -146,6 +154,7 @@ class _ChunkMisfit(torch.autograd.Function):
         return (f[0] / cascade.data_size).to(torch.float32)
 
     @staticmethod
+    @once_differentiable
     def backward(ctx, g):
         x, prb, pos, mag, data = ctx.saved_tensors
         cascade = ctx.cascade

@@ -389,3 +389,18 @@ def test_fidelity_from_two_threads():
     for got, ref in zip(res, refs):
         for a, b in zip(got, ref):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("fused", [True, False])
+@pytest.mark.parametrize("wrt", [0, 1, 2])
+def test_second_derivatives_are_refused(fused, wrt):
+    """A derivative of the data term's gradients, whose main terms autograd cannot
+    see, raises instead of giving the rest."""
+    fid, args = _small_fidelity(n=32, ntheta=3)
+    if not fused:
+        fid._use_fused = lambda *a: False
+    t = [a.clone().requires_grad_() for a in args[:3]]
+    f = fid(*t, *args[3:])
+    g = torch.autograd.grad(f ** 2, t, create_graph=True)
+    with pytest.raises(RuntimeError, match="once_differentiable"):
+        (f + g[wrt].abs().sum()).backward()
