@@ -125,6 +125,21 @@ __device__ __forceinline__ float sample_y(const CascDims& D, float mag, float ry
   return (mag * (float)(ty - D.nz / 2) - ry + (mag - 1.0f) / 2.0f) + (float)(D.nzobj / 2);
 }
 
+// Whether tap j of a stencil at floor position i lies in [0, n), and its index
+// there.  Unsigned: an image shifted off the object by more than an int holds
+// puts i at the type's limit, where i + 1 would overflow into the range.
+__device__ __forceinline__ bool tap_in(int i, int j, int n, int& at) {
+  const unsigned r = (unsigned)i + (unsigned)(j - 1);
+  at = r < (unsigned)n ? (int)r : 0;
+  return r < (unsigned)n;
+}
+
+// A shift with infinity held to 1e30, as far off any object: ColGeo subtracts a
+// position from its floor, which has no value at infinity.  NaN stays NaN.  (Held
+// per row: holding each pixel's position takes the forward rows of 720 images of
+// 128^2 from 95 us to 103.)
+__device__ __forceinline__ float finite_shift(float r) { return isinf(r) ? copysignf(1e30f, r) : r; }
+
 // Vertical stencil of one detector row: the four object rows it reads
 // (clamped into range; taps outside the object get weight 0) and their
 // weights.  The whole detector row shares it.
@@ -141,9 +156,7 @@ struct RowGeo {
     if (ORDER >= 2) bw2(dy, d2py);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int r = iy + j - 1;
-      const bool in = r >= 0 && r < D.nzobj;
-      yy[j] = in ? r : 0;
+      const bool in = tap_in(iy, j, D.nzobj, yy[j]);
       if (!in) {
         py[j] = 0.f;
         if (ORDER >= 1) dpy[j] = 0.f;
@@ -188,9 +201,7 @@ struct ColGeoEdge {
     if (ORDER >= 2) bw2(dx, d2px);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int c = ix + j - 1;
-      const bool in = c >= 0 && c < D.nobj;
-      xx[j] = in ? c : 0;
+      const bool in = tap_in(ix, j, D.nobj, xx[j]);
       if (!in) {
         px[j] = 0.f;
         if (ORDER >= 1) dpx[j] = 0.f;
@@ -360,6 +371,7 @@ k_casc_fwd(const T* __restrict__ c, const float* __restrict__ pos, const float* 
   T* V = reinterpret_cast<T*>(reinterpret_cast<char*>(smem) + CF::FFT_BYTES) + (long)line * (D.nobj + 2 * kVPad);
   const float m0 = valid ? mag[img] : 1.f;
   const float2 r = valid ? ld_pos(pos, img) : make_float2(0.f, 0.f);
+  const float rx = finite_shift(r.y);
   const RowGeo<0> rg(D, m0, r.x, ty);
   if (valid) {
     const float* const w[1] = {rg.py};
@@ -369,7 +381,7 @@ k_casc_fwd(const T* __restrict__ c, const float* __restrict__ pos, const float* 
   for (int tx = t; tx < N; tx += TT) {
     float2 u = make_float2(0.f, 0.f);
     if (valid) {
-      const ColGeo<0> cg(D, m0, r.y, tx);
+      const ColGeo<0> cg(D, m0, rx, tx);
       T v[4];
       vrow4(V, cg.x0, v);
       const T x22 = dot4(cg.px, v);
@@ -673,6 +685,7 @@ k_casc_adj(const float2* __restrict__ tmp, float2* __restrict__ Pc, T* __restric
   SmRow sm{smem + line * SmRow::padded(N)};
   const float m0 = valid ? mag[img] : 1.f;
   const float2 r = valid ? ld_pos(pos, img) : make_float2(0.f, 0.f);
+  const float rx = finite_shift(r.y);
   const RowGeo<2> rg(D, m0, r.x, ty);
   if (valid) {
     const float* const w[3] = {rg.py, rg.dpy, rg.d2py};
@@ -689,7 +702,7 @@ k_casc_adj(const float2* __restrict__ tmp, float2* __restrict__ Pc, T* __restric
     Yr[i] = make_float2(0.f, 0.f);
     if (!valid) continue;
     const float2 G = sm.ld(dct_perm(tx, N));
-    const ColGeo<2> cg(D, m0, r.y, tx);
+    const ColGeo<2> cg(D, m0, rx, tx);
     T x22 = El<T>::zero(), ax = El<T>::zero(), hxx = El<T>::zero();
     T ay = El<T>::zero(), hxy = El<T>::zero(), hyy = El<T>::zero();
 #pragma unroll
@@ -738,7 +751,7 @@ k_casc_adj(const float2* __restrict__ tmp, float2* __restrict__ Pc, T* __restric
     const int ixw = (int)floorf(x);
     float w[4];
     bw0(x - (float)ixw, w);
-    tcol[tx] = ixw - 1;
+    tcol[tx] = (int)((unsigned)ixw - 1u);
 #pragma unroll
     for (int j = 0; j < 4; ++j) twt[j * N + tx] = w[j];
   }

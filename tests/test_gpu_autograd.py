@@ -404,3 +404,18 @@ def test_second_derivatives_are_refused(fused, wrt):
     g = torch.autograd.grad(f ** 2, t, create_graph=True)
     with pytest.raises(RuntimeError, match="once_differentiable"):
         (f + g[wrt].abs().sum()).backward()
+
+
+@pytest.mark.parametrize("far", [float("inf"), -float("inf"), 1e30, -1e30, 4000.0, -33.0])
+@pytest.mark.parametrize("axis", [0, 1])
+def test_fidelity_of_an_image_far_off_the_object(far, axis):
+    """An image shifted off the object, infinitely far included, sees its zeros: the
+    fused term's value and gradients against the composition's."""
+    fid, args = _small_fidelity()
+    args[2][1, 0, axis] = far
+    fused = _value_and_grads(fid, args)
+    assert fid._use_fused(*args, False)
+    fid._use_fused = lambda *a: False
+    for a, b in zip(fused, _value_and_grads(fid, args)):
+        assert torch.isfinite(torch.view_as_real(a) if a.is_complex() else a).all()
+        assert rel_l2(a.cpu().numpy(), b.cpu().numpy()) < 1e-5

@@ -526,3 +526,25 @@ def test_bh_checkpoints_hold_the_iteration_state(golden, tmp_path):
     assert ck["iter"] == 2
     for k in ("obj", "prb", "pos"):
         assert rel_l2(ck[k].numpy(), states[1][k]) < 1e-6, k
+
+
+@pytest.mark.parametrize("axis", [0, 1])
+def test_cascade_of_an_image_shifted_off_the_object(golden, axis):
+    """However far off the object an image is shifted, infinity included, it sees
+    the object's zeros: the objective, the gradients and the Hessian forms of one
+    shifted off by 4000 pixels, to the bit."""
+    rec, v, gr, et = _cascade_setup(golden("rec"))
+
+    def terms(far):
+        v["pos"][1, 0, axis] = far
+        out = {k: torch.zeros_like(v[k]) for k in v}
+        rec.gradients_cascade(v, out)
+        return [rec.min(v["prb"], None, v["pos"], v["proj"]), rec.hessian_cascade(v, gr, et),
+                rec.hessian_cascade(v, et, et)], out
+    ref, gref = terms(4000.0)
+    assert np.isfinite(ref).all() and not gref["pos"][1, 0].any()
+    for far in (-4000.0, 3e9, -3e9, 1e30, -1e30, float("inf"), -float("inf")):
+        got, out = terms(far)
+        assert got == ref, (far, got, ref)
+        for k in out:
+            assert torch.equal(out[k], gref[k]), (far, k)
