@@ -1283,6 +1283,7 @@ extern "C" int ht_rec_create(int n, int nz, int nobj, int nzobj, int ntheta, int
   const cudaError_t e = cudaMalloc(&base, rec_layout(&r, nullptr));
   if (e != cudaSuccess) {
     set_error(std::string("ht_rec_create: ") + cudaGetErrorString(e));
+    cudaGetLastError();  // the next launch's check must not find this call's failure
     return kCudaError;
   }
   r.owned = base;

@@ -42,6 +42,16 @@ from . import _lib
 from .rec import Rec
 
 
+def radon_slices(n, nz):
+    """Slices the Radon workspace of an [nz, n, n] volume holds (csrc/tomo.cu): what
+    runs together is rounded up to the slices interleaved (4, 8 or 16); at 1024^2
+    and above up to four slices past a multiple of 16 run by themselves in the same
+    room."""
+    run = nz - nz % 16 if n >= 1024 and nz > 16 and nz % 16 <= 4 else nz
+    zi = 16 if run > 8 else (8 if run > 4 else 4)
+    return -(-run // zi) * zi
+
+
 def estimate_bytes(args):
     """Device bytes one reconstruction of these sizes holds: the arrays of
     Rec (vars/grads/etas, coefficients, data), the fused-cascade workspace,
@@ -54,8 +64,7 @@ def estimate_bytes(args):
     total = 3 * obj + 7 * proj                                  # obj x3; proj, coefficients, gradient x7
     total += img * 4 + 4 * ndist * nz * n * c8                  # data, probe arrays
     total += 3 * img * c8 + max(img, ntheta * ndist * nz * nobj) * c8   # x0, P, two spectra / S^T rows
-    zb = 8 if 2 * nobj <= 1024 else (4 if 2 * nobj == 2048 else 2)
-    nzp = -(-nzobj // zb) * zb
+    nzp = radon_slices(nobj, nzobj)
     total += nzp * 6 * nobj * nobj * c8 + nzp * ntheta * nobj * c8   # Radon workspace
     total += ndist * 4 * nz * n * c8 + ndist * nz * n * c8          # Fresnel tables
     return int(total * 1.1) + (64 << 20)

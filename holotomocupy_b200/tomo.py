@@ -71,8 +71,18 @@ class Tomo:
                      torch.from_numpy(phi).to(self.device))
         h = ctypes.c_void_p()
         with torch.cuda.device(self.device):
-            _lib.call("ht_tomo_create", n, nz, self.ntheta, theta.ctypes.data_as(ctypes.c_void_p),
-                      phi.ctypes.data_as(ctypes.c_void_p), ctypes.byref(h))
+            while True:
+                try:
+                    _lib.call("ht_tomo_create", n, self._nz, self.ntheta, theta.ctypes.data_as(ctypes.c_void_p),
+                              phi.ctypes.data_as(ctypes.c_void_p), ctypes.byref(h))
+                    break
+                except _lib.HoloError as e:
+                    # the workspace is rounded up to 4, 8 or 16 slices: where it has no
+                    # room so, the whole groups of the slices, taken slab by slab
+                    less = nz - nz % 16 if nz >= 16 else nz // 8 * 8
+                    if "out of memory" not in str(e) or not 0 < less < self._nz:
+                        raise
+                    self._nz = less
         self._h = h
         self._filters = {}
 
@@ -124,12 +134,13 @@ class Tomo:
                               _lib.ptr(sym) if sym is not None else None, float(scale), st)
         return res
 
-    def _result(self, out, x, shape, nz):
+    @staticmethod
+    def _result(out, x, shape):
         """(the array the kernels write, whether out still has to be copied from
-        it) for an operator on the contiguous x of nz slices.  out itself is written where it
+        it) for an operator on the contiguous x.  out itself is written where it
         is an array of the result's type and layout on x's device; any other out
         (on the host or another GPU, strided, of another type) is copied into, and
-        so is one that overlaps x when the volume takes several slabs, whose later
+        so is one that overlaps x: of a volume that runs in several parts, the later
         ones would read what the earlier ones wrote."""
         if out is not None and not (out.is_conj() or out.is_neg()):
             real, size = not x.is_complex(), math.prod(shape)
@@ -137,7 +148,7 @@ class Tomo:
                     and (tuple(out.shape) == shape and not out.requires_grad if real else out.numel() == size))
             a, b, width = x.data_ptr(), out.data_ptr(), x.element_size()
             apart = a + x.numel() * width <= b or b + size * width <= a
-            if fits and (apart or nz <= self._nz):
+            if fits and apart:
                 if not out.is_inference():
                     torch.autograd.graph.increment_version(out)
                 return out, False
@@ -151,7 +162,7 @@ class Tomo:
         if tuple(obj.shape[1:]) != (self.n, self.n):
             raise ValueError(f"obj must be [nz, {self.n}, {self.n}], got {tuple(obj.shape)}")
         x = obj.to(torch.complex64 if obj.is_complex() else torch.float32).contiguous().resolve_neg()
-        res, copy = self._result(out, x, (self.ntheta, nz, self.n), nz)
+        res, copy = self._result(out, x, (self.ntheta, nz, self.n))
         self._R_into(x, res)
         return out.copy_(res) if copy else res
 
@@ -165,7 +176,7 @@ class Tomo:
         if data.shape[0] != self.ntheta or data.shape[2] != self.n:
             raise ValueError(f"data must be [{self.ntheta}, nz, {self.n}], got {tuple(data.shape)}")
         x = data.to(torch.complex64 if data.is_complex() else torch.float32).contiguous().resolve_neg()
-        res, copy = self._result(out, x, (nz, self.n, self.n), nz)
+        res, copy = self._result(out, x, (nz, self.n, self.n))
         self._RT_into(x, res, scale=scale, sym=sym)
         return out.copy_(res) if copy else res
 

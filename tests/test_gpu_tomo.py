@@ -228,3 +228,72 @@ def test_R_RT_out_over_the_input(dtype, capacity):
         big = torch.cat([x.reshape(-1), x.reshape(-1)[:5]])
         view = big[5:].view(n, n, n)
         assert torch.equal(op(big[:n ** 3].view(n, n, n), out=view), ref)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "complex64"])
+@pytest.mark.parametrize("nz", [17, 20, 21])
+def test_R_RT_remainder_run_at_1024(dtype, nz):
+    """Up to four slices past a multiple of 16 run by themselves at 1024^2: the
+    slices of a call of them alone, in volumes taller than the call too."""
+    from holotomocupy_b200 import Tomo
+    n, ntheta = 1024, 7
+    theta = np.linspace(0, np.pi, ntheta, endpoint=False).astype("float32")
+    g = torch.Generator(device="cuda").manual_seed(nz)
+    dt = getattr(torch, dtype)
+    x = torch.randn(nz, n, n, dtype=dt, device="cuda", generator=g)
+    y = torch.randn(ntheta, nz, n, dtype=dt, device="cuda", generator=g)
+    t, one, part = Tomo(n, nz, theta, 0.9), Tomo(n, 16, theta, 0.9), Tomo(n, 18, theta, 0.9)
+    for op, a, ax in (("R", x, 0), ("RT", y, 1)):
+        pieces = [getattr(one, op)(a.narrow(ax, z, min(16, nz - z)).contiguous()) for z in (0, 16)]
+        ref = torch.cat(pieces, dim=1 - ax)
+        for tomo in (t, part):   # 18 slices of capacity: 16 + 2 of the call, then the rest
+            got = getattr(tomo, op)(a)
+            assert rel_l2(got.cpu().numpy(), ref.cpu().numpy()) < 1e-6
+            # the last slice alone: its error is not hidden by the others'
+            assert rel_l2(got.select(1 - ax, nz - 1).cpu().numpy(), ref.select(1 - ax, nz - 1).cpu().numpy()) < 1e-6
+
+
+@pytest.mark.parametrize("n,nz", [(256, 17), (256, 24), (1024, 9), (1024, 20), (1024, 21)])
+def test_workspace_slices(n, nz):
+    """The memory a Tomo takes beyond one of four slices is that of the slices
+    serving counts."""
+    from holotomocupy_b200 import Tomo
+    from holotomocupy_b200.serving import radon_slices
+    theta = np.linspace(0, np.pi, 64, endpoint=False).astype("float32")
+
+    def held(nz):
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0] + torch.cuda.memory_reserved()
+        t = Tomo(n, nz, theta, 0.9)
+        return free - torch.cuda.mem_get_info()[0] - torch.cuda.memory_reserved(), t
+    base, _ = held(4)
+    got, _ = held(nz)
+    want = (radon_slices(n, nz) - 4) * (6 * n + 64) * n * 8
+    assert abs(got - base - want) < 0.02 * want + (8 << 20)   # allocations come in 2 MiB pages
+
+
+@pytest.mark.parametrize("n,nz,less", [(32, 20, 16), (32, 13, 8)])
+def test_tomo_without_room_for_the_rounded_workspace(monkeypatch, n, nz, less):
+    """Where the workspace of all slices has no room, the whole groups of them run
+    slab by slab; another failure, and one of the smallest group, is raised."""
+    from holotomocupy_b200 import Tomo, _lib
+    theta = np.linspace(0, np.pi, 12, endpoint=False).astype("float32")
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn(nz, n, n, dtype=torch.complex64, device="cuda", generator=g)
+    ref = Tomo(n, nz, theta, 0.9).R(x)
+    call = _lib.call
+
+    def failing(limit, message):
+        def f(name, *args):
+            if name == "ht_tomo_create" and args[1] > limit:
+                raise _lib.HoloError(f"{name} failed with status 2: {message}")
+            return call(name, *args)
+        return f
+    monkeypatch.setattr(_lib, "call", failing(less, "ht_tomo_create: out of memory"))
+    t = Tomo(n, nz, theta, 0.9)
+    assert t._nz == less
+    assert rel_l2(t.R(x).cpu().numpy(), ref.cpu().numpy()) < 1e-6
+    for limit, message in ((less - 1, "out of memory"), (less, "unknown error")):
+        monkeypatch.setattr(_lib, "call", failing(limit, message))
+        with pytest.raises(_lib.HoloError, match=message):
+            Tomo(n, nz, theta, 0.9)

@@ -5,7 +5,7 @@ import types
 
 import numpy as np
 
-from holotomocupy_b200.serving import args_key, estimate_bytes
+from holotomocupy_b200.serving import args_key, estimate_bytes, radon_slices
 from holotomocupy_b200.synthetic import workload_args
 
 
@@ -36,3 +36,16 @@ def test_estimate_grows_with_the_problem():
     assert 0 < small < large
     # n^4 work, n^3-and-more memory: a 512^3 x 900 x 4 reconstruction needs tens of GB
     assert 40e9 < estimate_bytes(workload_args(512, 900, 4)) < 120e9
+
+
+def test_estimate_counts_the_radon_workspace_slices():
+    """Slices are interleaved by 4, 8 or 16 at every size; from 1024^2 on a short
+    remainder runs in the room of the others (tests/test_gpu_tomo.py compares
+    these numbers with the memory a Tomo takes)."""
+    assert [radon_slices(256, nz) for nz in (1, 4, 5, 8, 9, 16, 17, 24, 33)] == [4, 4, 8, 8, 16, 16, 32, 32, 48]
+    assert [radon_slices(2048, nz) for nz in (1, 9, 16, 17, 20, 21, 31, 36, 37)] == [4, 16, 16, 16, 16, 32, 32, 32, 48]
+    a, b = workload_args(128, 224, 4), workload_args(128, 224, 4)
+    a.nzobj, b.nzobj = 16, 17
+    a.nobj = b.nobj = 512
+    one = 512 * 512 * 8 * 3 + 224 * 512 * 8 * 7   # one more slice of the arrays
+    assert estimate_bytes(b) - estimate_bytes(a) > 1.09 * (one + 16 * (6 * 512 * 512 + 224 * 512) * 8)
