@@ -100,7 +100,9 @@ typedef struct ht_tomo_s ht_tomo_s;
  * theta_host: host float32 [ntheta]; phi_host: host float32 [n, n], the
  * reference's deapodisation factor already multiplied by the support mask
  * and 1/(n sqrt(n ntheta)) (tomo.py:19-21, 34-47).  The handle owns a
- * workspace of nz*(6n^2) + ntheta*nz*n complex64 samples. */
+ * workspace of nz*(6n^2) + ntheta*nz*n complex64 samples, nz rounded up to the
+ * slices interleaved (4, 8 or 16; from n = 1024 on up to four slices past a
+ * multiple of 16 are not counted).  obj and sino of a call must not overlap. */
 int ht_tomo_create(int n, int nz, int ntheta, const float* theta_host, const float* phi_host, ht_tomo_s** out);
 int ht_tomo_destroy(ht_tomo_s* t);
 

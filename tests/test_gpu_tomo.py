@@ -297,3 +297,19 @@ def test_tomo_without_room_for_the_rounded_workspace(monkeypatch, n, nz, less):
         monkeypatch.setattr(_lib, "call", failing(limit, message))
         with pytest.raises(_lib.HoloError, match=message):
             Tomo(n, nz, theta, 0.9)
+
+
+@pytest.mark.parametrize("n,ntheta", [(64, 300), (64, 90), (128, 401)])
+def test_R_RT_over_a_full_turn(n, ntheta):
+    """Angles over 2 pi, sorted and not: theta and theta + pi share a line from
+    opposite ends."""
+    from holotomocupy_b200 import Tomo
+    rng = np.random.default_rng(ntheta)
+    theta = np.linspace(0, 2 * np.pi, ntheta, endpoint=False)
+    theta = (rng.permutation(theta) if ntheta % 2 else theta).astype("float32")
+    nz = 9
+    t, o = Tomo(n, nz, theta, 1), O.Tomo(n, nz, theta, 1, "complex64")
+    x = (rng.standard_normal((nz, n, n)) + 1j * rng.standard_normal((nz, n, n))).astype("complex64")
+    y = (rng.standard_normal((ntheta, nz, n)) + 1j * rng.standard_normal((ntheta, nz, n))).astype("complex64")
+    assert rel_l2(t.R(torch.from_numpy(x).cuda()).cpu().numpy(), o.R(x)) < TOL
+    assert rel_l2(t.RT(torch.from_numpy(y).cuda()).cpu().numpy(), o.RT(y)) < TOL
