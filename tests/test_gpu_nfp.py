@@ -97,3 +97,38 @@ def test_nfp_graph_iteration_matches_host(golden):
     np.testing.assert_allclose(h1, h0, rtol=1e-9)
     for k in v0:
         assert rel_l2(v1[k], v0[k]) < 1e-6, k
+
+
+@pytest.mark.parametrize("dt", ["complex64", "float32"])
+@pytest.mark.parametrize("nimg", [1, 2, 31, 70, 97])
+def test_shared_coefficients_gradient_over_groups(dt, nimg):
+    """The gradient of one coefficient array under all images, summed in groups
+    whose last one may not be full, against the sum of the gradients of as many
+    separate arrays; the other gradients to the bit."""
+    import ctypes
+
+    from holotomocupy_b200 import Propagation, _lib
+    n, nobj = 32, 48
+    rng = np.random.default_rng(nimg)
+    real = lambda *s: rng.standard_normal(s).astype("float32")
+    c = real(nobj, nobj) if dt == "float32" else (real(nobj, nobj) + 1j * real(nobj, nobj)).astype("complex64")
+    c = cuda(0.1 * c)
+    prb = cuda((1 + 0.1 * real(1, n, n) + 0.1j * real(1, n, n)).astype("complex64"))
+    pos, mag = cuda(4 * real(nimg, 1, 2)), torch.ones(nimg, 1, device="cuda")
+    data = cuda(1 + 0.1 * real(nimg, 1, n, n))
+    prop = Propagation(n, n, nimg, 1, 7.3e-11, 20e-9, [3e-3])
+    out = []
+    for shared in (1, 0):
+        h = ctypes.c_void_p()
+        _lib.call("ht_rec_create", n, n, nobj, nobj, nimg, 1, int(dt == "complex64"), prop._h, ctypes.byref(h))
+        _lib.call("ht_rec_set_shared_coefficients", h, shared)
+        cs = c if shared else c.expand(nimg, nobj, nobj).contiguous()
+        gc, gpos, gprb = torch.empty_like(cs), torch.empty_like(pos), torch.empty_like(prb)
+        _lib.call("ht_rec_gradient", h, _lib.ptr(cs), _lib.ptr(pos), _lib.ptr(mag), _lib.ptr(prb), _lib.ptr(data),
+                  _lib.ptr(gc), _lib.ptr(gpos), _lib.ptr(gprb), None, 1.0, 1.0, 0, _lib.stream_ptr())
+        torch.cuda.synchronize()
+        _lib.lib().ht_rec_destroy(h)
+        wide = torch.complex128 if gc.is_complex() else torch.float64
+        out.append((gc.to(wide) if shared else gc.to(wide).sum(0), gpos, gprb))
+    assert rel_l2(out[0][0].cpu().numpy(), out[1][0].cpu().numpy()) < 1e-6
+    assert torch.equal(out[0][1], out[1][1]) and torch.equal(out[0][2], out[1][2])

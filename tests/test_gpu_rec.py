@@ -548,3 +548,28 @@ def test_cascade_of_an_image_shifted_off_the_object(golden, axis):
         assert got == ref, (far, got, ref)
         for k in out:
             assert torch.equal(out[k], gref[k]), (far, k)
+
+
+@pytest.mark.parametrize("mode", ["host", "graph"])
+@pytest.mark.parametrize("niter", [0, 1, 4, 64])
+def test_proj_arrays_after_bh_are_R_of_the_objects(golden, mode, niter):
+    """vars, grads and etas proj, formed at the end of BH from the coefficients
+    the iterations kept, against R of the arrays' objects.  R and the spline
+    differ by their own rounding (5e-7), and each iteration adds a rounded
+    product and sum (1.2e-7) to the coefficients and to the object."""
+    from holotomocupy_b200.rec import Rec
+    g = golden("rec")
+    n, ntheta, ndist, nobj, _ = [int(v) for v in g["bh_dims"]]
+    rec = Rec(rec_args(n, ntheta, ndist, nobj, niter))
+    rec.data[:] = cuda(g["bh_data"])
+    rec.vars["obj"][:] = cuda(0.5 * g["bh_obj_true"])
+    rec.vars["prb"][:] = 1
+    rec.vars["pos"][:] = cuda(g["bh_pos_true"] + g["bh_pos_err"])
+    rec.BH(mode=mode)
+    for name, d, scale in (("vars", rec.vars, rec.norm_const), ("grads", rec.grads, 1.0), ("etas", rec.etas, 1.0)):
+        ref = rec.cl_tomo.R(d["obj"] / scale).cpu().numpy()
+        got = d["proj"].cpu().numpy()
+        if niter == 0 and name != "vars":
+            assert not got.any() and not ref.any()
+            continue
+        assert rel_l2(got, ref) < 5e-7 + 2 * 1.2e-7 * niter, (name, rel_l2(got, ref))

@@ -313,3 +313,46 @@ def test_R_RT_over_a_full_turn(n, ntheta):
     y = (rng.standard_normal((ntheta, nz, n)) + 1j * rng.standard_normal((ntheta, nz, n))).astype("complex64")
     assert rel_l2(t.R(torch.from_numpy(x).cuda()).cpu().numpy(), o.R(x)) < TOL
     assert rel_l2(t.RT(torch.from_numpy(y).cuda()).cpu().numpy(), o.RT(y)) < TOL
+
+
+@pytest.mark.parametrize("dtype", ["float32", "complex64"])
+@pytest.mark.parametrize("n,ntheta,nz,slab", [(32, 100, 5, 4), (48, 33, 8, 8), (64, 150, 9, 4), (96, 31, 17, 16),
+                                              (64, 48, 20, 8)])
+def test_R_RT_fbp_over_types_and_slabs(dtype, n, ntheta, nz, slab):
+    """Real and complex volumes, whole and by slabs, at slice counts around the
+    interleaves: R, R^T and filtered back-projection against the FP64 oracle,
+    a real volume's as the real part of a complex one's."""
+    from holotomocupy_b200 import Tomo
+    rng = np.random.default_rng(n + nz)
+    theta = np.linspace(0, np.pi, ntheta, endpoint=False).astype("float32")
+    x, y = rng.standard_normal((nz, n, n)), rng.standard_normal((ntheta, nz, n))
+    if dtype == "complex64":
+        x, y = x + 1j * rng.standard_normal(x.shape), y + 1j * rng.standard_normal(y.shape)
+    x, y = x.astype(dtype), y.astype(dtype)
+    wide = np.complex128 if dtype == "complex64" else np.float64
+    o = O.Tomo(n, nz, theta, 0.9, "complex128")
+    refs = [o.R(x.astype(wide)), o.RT(y.astype(wide))]
+    refs += [o.fbp(y.astype(wide), f) for f in ("ramp", "shepp", "parzen")]
+    for t in (Tomo(n, nz, theta, 0.9), Tomo(n, slab, theta, 0.9)):
+        xt, yt = torch.from_numpy(x).cuda(), torch.from_numpy(y).cuda()
+        got = [t.R(xt), t.RT(yt)] + [t.fbp(yt, f) for f in ("ramp", "shepp", "parzen")]
+        for a, b in zip(got, refs):
+            assert a.dtype == xt.dtype and rel_l2(a.cpu().numpy(), b) < TOL
+        if dtype == "float32":
+            assert rel_l2(t.R(xt.to(torch.complex64)).real.cpu().numpy(), got[0].cpu().numpy()) < 1e-7
+            assert rel_l2(t.RT(yt.to(torch.complex64)).real.cpu().numpy(), got[1].cpu().numpy()) < 1e-7
+
+
+@pytest.mark.parametrize("dtype", ["float32", "complex64"])
+@pytest.mark.parametrize("n", [18, 96, 512])
+def test_filter_sino_matches_oracle(dtype, n):
+    """The detector filter alone (ht_filter_rows)."""
+    from holotomocupy_b200 import Tomo
+    theta = np.linspace(0, np.pi, 5, endpoint=False).astype("float32")
+    rng = np.random.default_rng(n)
+    d = rng.standard_normal((5, 3, n))
+    d = (d + 1j * rng.standard_normal(d.shape) if dtype == "complex64" else d).astype(dtype)
+    t, o = Tomo(n, 3, theta, 1), O.Tomo(n, 3, theta, 1, "complex128")
+    for f in ("ramp", "shepp", "parzen"):
+        got = t._filter_sino(torch.from_numpy(d).cuda(), f)
+        assert rel_l2(got.cpu().numpy(), o.filter_sino(d.astype(np.complex128 if dtype == "complex64" else float), f)) < 1e-6
