@@ -500,7 +500,7 @@ k_casc_resid512(float2* __restrict__ tmp, float2* __restrict__ x0c, const float*
         x0c[row * N + tx] = x0;
         // rec_mpi.py:557-559: scale * (x - y * (x / |x|))
         float2 l = make_float2(x0.x / a, x0.y / a);
-          if (D.zero_grad && a == 0.f) l = make_float2(0.f, 0.f);
+        if (D.zero_grad && a == 0.f) l = make_float2(0.f, 0.f);
         v[i] = make_float2(scale * (x0.x - d * l.x), scale * (x0.y - d * l.y));
       }
     }
@@ -733,12 +733,12 @@ k_casc_adj(const float2* __restrict__ tmp, float2* __restrict__ Pc, T* __restric
   double v[5];
 #pragma unroll
   for (int i = 0; i < 5; ++i) v[i] = s[i];
-  line_sums<TT, 5>(v, red, line, t);  // contains barriers: G is no longer read
+  line_sums<TT, 5>(v, red, line, t);
   if (t == 0 && valid) {
 #pragma unroll
     for (int i = 0; i < 5; ++i) rows[row * 5 + i] = v[i];  // per-image sums: k_rows_img
   }
-  __syncthreads();
+  __syncthreads();  // G and V are no longer read
   // Y22 into the FFT line; per detector pixel its stencil's first column + 1
   // and tap weights into the gather tables (over V, which is consumed)
   int* tcol = reinterpret_cast<int*>(V);

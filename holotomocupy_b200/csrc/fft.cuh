@@ -360,6 +360,7 @@ __device__ __forceinline__ void fft_stage(float2 (&v)[E], const SM& sm, int t,
   constexpr int NR = N / R;
   static_assert(E % R == 0, "radix must divide the samples per thread");
   static_assert(R <= 8 || R == 16, "twiddles() covers radices up to 8, and 16");
+  static_assert(!load_half<SM>::value || R % 4 == 0, "a central-half view's ld has no sample outside the half");
 #pragma unroll
   for (int s = 0; s < NB; ++s) {
     const int b = t + s * T;

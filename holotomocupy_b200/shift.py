@@ -40,7 +40,7 @@ class Shift:
         h = ctypes.c_void_p()
         with torch.cuda.device(self.device):
             _lib.call("ht_shift_create", n, npsi, nz, nzpsi, 1 if self._complex else 0, ctypes.byref(h))
-            # the prefilter always runs on complex samples
+            # a complex-sample handle as well: real objects' coeffback, Sback and prefilter go through it
             hc = ctypes.c_void_p()
             _lib.call("ht_shift_create", n, npsi, nz, nzpsi, 1, ctypes.byref(hc))
         self._h, self._hc = h, hc
