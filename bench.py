@@ -956,8 +956,8 @@ KERNEL_BYTES = {
     "k_dct_cols": lambda r: 16 * r.nz * r.n,
     # the Fourier-grid disc the polar samples reach (radius n + m) read; sinogram rows written
     "k_tgather": lambda r: 8 * np.pi * (r.nobj + 4) ** 2 + 8 * r.ntheta * r.nobj,
-    # sinogram spectra read; the 2n x 2n Fourier grid written
-    "k_tcell": lambda r: 8 * r.ntheta * r.nobj + 32 * r.nobj ** 2,
+    # sinogram spectra read; the Fourier-grid cells the transform keeps (radius n + 16) written
+    "k_tcell": lambda r: 8 * r.ntheta * r.nobj + 8 * np.pi * (r.nobj + 16) ** 2,
 }
 # (dram__bytes_read.sum + dram__bytes_write.sum) of one captured launch, its
 # work units and the case it ran on; traffic at other sizes is this ratio to
@@ -973,8 +973,8 @@ NCU_CAPTURE = {
     "k_casc_hess_fwd": (3.426991e9, 2 * 384, _CASE_512_96),
     "k_casc_hess_q": (2.828069e9, 2 * 384, _CASE_512_96),
     "k_dct_cols": (1.569036e9, 384, _CASE_512_96),
-    "k_tgather": (0.651061e9, 256, _CASE_256_448),
-    "k_tcell": (0.797557e9, 256, _CASE_256_448),   # the pair lists come from DRAM once (group-major block order)
+    "k_tgather": (0.647618e9, 256, _CASE_256_448),
+    "k_tcell": (0.706639e9, 256, _CASE_256_448),   # the lists come from DRAM once (group-major block order)
 }
 
 
