@@ -74,7 +74,7 @@ SIGNATURES = {
     "ht_rec_workspace_bytes": [_c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _vp, _c_int,
                                ctypes.POINTER(ctypes.c_size_t)],
     "ht_rec_create_in": [_c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _vp, _c_int, _vp, ctypes.c_size_t,
-                         ctypes.POINTER(_vp)],
+                         _c_double, _c_int, ctypes.POINTER(_vp)],
     "ht_rec_destroy": [_vp],
     "ht_rec_forward": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
     "ht_rec_gradient": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _c_float, _c_float, _c_int, _vp],

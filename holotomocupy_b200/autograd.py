@@ -115,6 +115,7 @@ class _Cascade:
         self.data_size = term.data_size
         self.sizes = (term.n, term.nz, term.nobj, term.nzobj, ntheta, term.ndist,
                       int(term.sh.obj_dtype == "complex64"))
+        self.bytes = term._workspace_bytes
 
     def coeff(self, x):
         return self.sh.coeff(x if self.tomo is None else self.tomo.R(x.contiguous()))
@@ -122,14 +123,16 @@ class _Cascade:
     @contextlib.contextmanager
     def handle(self, forward_only=False):
         with torch.cuda.device(self.sh.device):
-            size, h = ctypes.c_size_t(), ctypes.c_void_p()
-            args = (*self.sizes, self.prop._h, int(forward_only))
-            _lib.call("ht_rec_workspace_bytes", *args, ctypes.byref(size))
-            work = torch.empty(size.value, dtype=torch.uint8, device=self.sh.device)
-            _lib.call("ht_rec_create_in", *args, _lib.ptr(work), size.value, ctypes.byref(h))
+            key = self.sizes + (int(forward_only),)
+            size = self.bytes.get(key)
+            if size is None:
+                out = ctypes.c_size_t()
+                _lib.call("ht_rec_workspace_bytes", *self.sizes, self.prop._h, key[-1], ctypes.byref(out))
+                size = self.bytes[key] = out.value
+            work, h = torch.empty(size, dtype=torch.uint8, device=self.sh.device), ctypes.c_void_p()
+            _lib.call("ht_rec_create_in", *self.sizes, self.prop._h, key[-1], _lib.ptr(work), size,
+                      float(self.data_size), 1, ctypes.byref(h))   # 1: torch.abs has gradient 0 at 0
             try:
-                _lib.call("ht_rec_set_data_size", h, float(self.data_size))
-                _lib.call("ht_rec_set_zero_gradient", h, 1)   # torch.abs has gradient 0 at 0
                 yield h
             finally:
                 _lib.lib().ht_rec_destroy(h)
@@ -147,11 +150,11 @@ class _ChunkMisfit(torch.autograd.Function):
         ctx.cascade = cascade
         ctx.save_for_backward(x, prb, pos, mag, data)
         c = cascade.coeff(x)
-        f = torch.empty(1, dtype=torch.float64, device=x.device)
+        f = torch.empty((), dtype=torch.float64, device=x.device)
         with cascade.handle(forward_only=True) as h:
             _lib.call("ht_rec_forward", h, _lib.ptr(c), _lib.ptr(pos), _lib.ptr(mag), _lib.ptr(prb), _lib.ptr(data),
                       None, _lib.ptr(f), _lib.stream_ptr())
-        return (f[0] / cascade.data_size).to(torch.float32)
+        return (f / cascade.data_size).to(torch.float32)
 
     @staticmethod
     @once_differentiable
@@ -212,6 +215,7 @@ class DataFidelity(torch.nn.Module):
         self.bounds = [(a, min(a + self.chunk, self.ntheta)) for a in range(0, self.ntheta, self.chunk)]
         self.tomos = [Tomo(nobj, nzobj, theta[a:b], mask_r, norm_ntheta=self.ntheta) for a, b in self.bounds]
         self.sh, self.prop = sh, prop
+        self._workspace_bytes = {}   # of the fused cascade, by its sizes
 
     @classmethod
     def create(cls, n, nz, nobj, nzobj, theta, ndist, wavelength, voxelsize, distance, mask_r=None, chunk=None,

@@ -1305,7 +1305,8 @@ extern "C" int ht_rec_workspace_bytes(int n, int nz, int nobj, int nzobj, int nt
 }
 
 extern "C" int ht_rec_create_in(int n, int nz, int nobj, int nzobj, int ntheta, int ndist, int is_complex,
-                                ht_prop_s* prop, int forward_only, void* workspace, size_t bytes, ht_rec_s** out) {
+                                ht_prop_s* prop, int forward_only, void* workspace, size_t bytes, double ndata,
+                                int zero_gradient, ht_rec_s** out) {
   using namespace ht;
   HT_REQUIRE(out && workspace, "ht_rec_create_in: null pointer");
   ht_rec_s r;
@@ -1313,6 +1314,11 @@ extern "C" int ht_rec_create_in(int n, int nz, int nobj, int nzobj, int ntheta, 
   if (st != kOk) return st;
   HT_REQUIRE(reinterpret_cast<size_t>(workspace) % 512 == 0, "ht_rec_create_in: workspace must be 512-byte aligned");
   HT_REQUIRE(rec_layout(&r, static_cast<char*>(workspace)) <= bytes, "ht_rec_create_in: workspace too small");
+  r.D.zero_grad = zero_gradient ? 1 : 0;
+  if (ndata != 0.0) {
+    const int sd = ht_rec_set_data_size(&r, ndata);
+    if (sd != kOk) return sd;
+  }
   *out = new ht_rec_s(r);
   return kOk;
 }

@@ -233,11 +233,13 @@ int ht_rec_create(int n, int nz, int nobj, int nzobj, int ntheta, int ndist, int
 /* A handle in the caller's device memory (512-byte aligned, of at least
  * ht_rec_workspace_bytes bytes, kept until the handle's last call has run).  Makes
  * no device allocation and no synchronisation.  forward_only = 1: for
- * ht_rec_forward alone, in about a quarter of the memory. */
+ * ht_rec_forward alone, in about a quarter of the memory.  ndata: as for
+ * ht_rec_set_data_size (0: the handle's own); zero_gradient: as for
+ * ht_rec_set_zero_gradient. */
 int ht_rec_workspace_bytes(int n, int nz, int nobj, int nzobj, int ntheta, int ndist, int is_complex, ht_prop_s* prop,
                            int forward_only, size_t* bytes);
 int ht_rec_create_in(int n, int nz, int nobj, int nzobj, int ntheta, int ndist, int is_complex, ht_prop_s* prop,
-                     int forward_only, void* workspace, size_t bytes, ht_rec_s** out);
+                     int forward_only, void* workspace, size_t bytes, double ndata, int zero_gradient, ht_rec_s** out);
 int ht_rec_destroy(ht_rec_s* r);
 
 /* Forward model.  With amp != NULL: amp[ntheta, ndist, nz, n] = |x0|
