@@ -125,20 +125,22 @@ __device__ __forceinline__ float sample_y(const CascDims& D, float mag, float ry
   return (mag * (float)(ty - D.nz / 2) - ry + (mag - 1.0f) / 2.0f) + (float)(D.nzobj / 2);
 }
 
-// Whether tap j of a stencil at floor position i lies in [0, n), and its index
-// there.  Unsigned: an image shifted off the object by more than an int holds
-// puts i at the type's limit, where i + 1 would overflow into the range.
-__device__ __forceinline__ bool tap_in(int i, int j, int n, int& at) {
-  const unsigned r = (unsigned)i + (unsigned)(j - 1);
-  at = r < (unsigned)n ? (int)r : 0;
-  return r < (unsigned)n;
+// An image's magnification and shift (y, x), held to 5e5 and 1e9 (NaN stays NaN): a
+// sample's position is then finite and an int holds it with room for the taps (4096
+// rows at most).  A shift that was further off still lies off any object.
+__device__ __forceinline__ float held(float x, float lim) {
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x) : "f"(-lim));
+  asm("min.NaN.f32 %0, %0, %1;" : "+f"(x) : "f"(lim));
+  return x;
 }
-
-// A shift with infinity held to 1e30, as far off any object: ColGeo subtracts a
-// position from its floor, which has no value at infinity.  NaN stays NaN.  (Held
-// per row: holding each pixel's position takes the forward rows of 720 images of
-// 128^2 from 95 us to 103.)
-__device__ __forceinline__ float finite_shift(float r) { return isinf(r) ? copysignf(1e30f, r) : r; }
+__device__ __forceinline__ float ld_mag(const float* mag, long img) { return held(mag[img], 5e5f); }
+__device__ __forceinline__ float2 ld_pos(const float* pos, long img) {
+  return make_float2(pos[2 * img + 0], pos[2 * img + 1]);
+}
+__device__ __forceinline__ float2 ld_shift(const float* pos, long img) {
+  const float2 r = ld_pos(pos, img);
+  return make_float2(held(r.x, 1e9f), held(r.y, 1e9f));
+}
 
 // Vertical stencil of one detector row: the four object rows it reads
 // (clamped into range; taps outside the object get weight 0) and their
@@ -156,7 +158,9 @@ struct RowGeo {
     if (ORDER >= 2) bw2(dy, d2py);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const bool in = tap_in(iy, j, D.nzobj, yy[j]);
+      const int r = iy + j - 1;
+      const bool in = r >= 0 && r < D.nzobj;
+      yy[j] = in ? r : 0;
       if (!in) {
         py[j] = 0.f;
         if (ORDER >= 1) dpy[j] = 0.f;
@@ -201,7 +205,9 @@ struct ColGeoEdge {
     if (ORDER >= 2) bw2(dx, d2px);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const bool in = tap_in(ix, j, D.nobj, xx[j]);
+      const int c = ix + j - 1;
+      const bool in = c >= 0 && c < D.nobj;
+      xx[j] = in ? c : 0;
       if (!in) {
         px[j] = 0.f;
         if (ORDER >= 1) dpx[j] = 0.f;
@@ -217,10 +223,6 @@ __device__ __forceinline__ T dot4(const float (&w)[4], const T (&v)[4]) {
 #pragma unroll
   for (int j = 0; j < 4; ++j) El<T>::fma(a, w[j], v[j]);
   return a;
-}
-
-__device__ __forceinline__ float2 ld_pos(const float* pos, long img) {
-  return make_float2(pos[2 * img + 0], pos[2 * img + 1]);
 }
 
 // Doubles of shared scratch line_sums<T, K> needs for a block of THREADS,
@@ -369,9 +371,8 @@ k_casc_fwd(const T* __restrict__ c, const float* __restrict__ pos, const float* 
   const long th = img / D.ndist;
   SmRow sm{smem + line * SmRow::padded(N)};
   T* V = reinterpret_cast<T*>(reinterpret_cast<char*>(smem) + CF::FFT_BYTES) + (long)line * (D.nobj + 2 * kVPad);
-  const float m0 = valid ? mag[img] : 1.f;
-  const float2 r = valid ? ld_pos(pos, img) : make_float2(0.f, 0.f);
-  const float rx = finite_shift(r.y);
+  const float m0 = valid ? ld_mag(mag, img) : 1.f;
+  const float2 r = valid ? ld_shift(pos, img) : make_float2(0.f, 0.f);
   const RowGeo<0> rg(D, m0, r.x, ty);
   if (valid) {
     const float* const w[1] = {rg.py};
@@ -381,7 +382,7 @@ k_casc_fwd(const T* __restrict__ c, const float* __restrict__ pos, const float* 
   for (int tx = t; tx < N; tx += TT) {
     float2 u = make_float2(0.f, 0.f);
     if (valid) {
-      const ColGeo<0> cg(D, m0, rx, tx);
+      const ColGeo<0> cg(D, m0, r.y, tx);
       T v[4];
       vrow4(V, cg.x0, v);
       const T x22 = dot4(cg.px, v);
@@ -683,9 +684,8 @@ k_casc_adj(const float2* __restrict__ tmp, float2* __restrict__ Pc, T* __restric
   const int k = (int)(img % D.ndist);
   const long th = img / D.ndist;
   SmRow sm{smem + line * SmRow::padded(N)};
-  const float m0 = valid ? mag[img] : 1.f;
-  const float2 r = valid ? ld_pos(pos, img) : make_float2(0.f, 0.f);
-  const float rx = finite_shift(r.y);
+  const float m0 = valid ? ld_mag(mag, img) : 1.f;
+  const float2 r = valid ? ld_shift(pos, img) : make_float2(0.f, 0.f);
   const RowGeo<2> rg(D, m0, r.x, ty);
   if (valid) {
     const float* const w[3] = {rg.py, rg.dpy, rg.d2py};
@@ -702,7 +702,7 @@ k_casc_adj(const float2* __restrict__ tmp, float2* __restrict__ Pc, T* __restric
     Yr[i] = make_float2(0.f, 0.f);
     if (!valid) continue;
     const float2 G = sm.ld(dct_perm(tx, N));
-    const ColGeo<2> cg(D, m0, rx, tx);
+    const ColGeo<2> cg(D, m0, r.y, tx);
     T x22 = El<T>::zero(), ax = El<T>::zero(), hxx = El<T>::zero();
     T ay = El<T>::zero(), hxy = El<T>::zero(), hyy = El<T>::zero();
 #pragma unroll
@@ -751,7 +751,7 @@ k_casc_adj(const float2* __restrict__ tmp, float2* __restrict__ Pc, T* __restric
     const int ixw = (int)floorf(x);
     float w[4];
     bw0(x - (float)ixw, w);
-    tcol[tx] = (int)((unsigned)ixw - 1u);
+    tcol[tx] = ixw - 1;
 #pragma unroll
     for (int j = 0; j < 4; ++j) twt[j * N + tx] = w[j];
   }
@@ -837,8 +837,8 @@ k_casc_vsum(T* __restrict__ gc, const T* __restrict__ hbuf, const float* __restr
   for (int k = 0; k < D.ndist; ++k) {
     const long img = th * D.ndist + k;
     if (img >= D.nimg) break;  // the last group of a shared array's images
-    const float m0 = mag[img];
-    const float ry = pos[2 * img + 0];
+    const float m0 = ld_mag(mag, img);
+    const float ry = held(pos[2 * img + 0], 1e9f);
     const float C0 = -ry + (m0 - 1.0f) / 2.0f + (float)(D.nzobj / 2);
     int a0, a1, b0, b1;
     cand_range(m0, C0, iy0, D.nz / 2, D.nz, a0, a1);
@@ -920,8 +920,8 @@ k_casc_hess_fwd(const T* __restrict__ c, const float* __restrict__ pos, const fl
   SmRow sm0{smem + line * SmRow::padded(N)};
   SmRow sm1{smem + (LINES + line) * SmRow::padded(N)};
   const long coff = coef_off(D, th);
-  const float m0 = valid ? mag[img] : 1.f;
-  const float2 r = valid ? ld_pos(pos, img) : make_float2(0.f, 0.f);
+  const float m0 = valid ? ld_mag(mag, img) : 1.f;
+  const float2 r = valid ? ld_shift(pos, img) : make_float2(0.f, 0.f);
   const float2 rd0 = valid ? ld_pos(pos0, img) : make_float2(0.f, 0.f);
   const float2 rd1 = (valid && NDIR == 2) ? ld_pos(pos1, img) : make_float2(0.f, 0.f);
   // P streams from DRAM: each pixel's value is loaded one pixel ahead (the
