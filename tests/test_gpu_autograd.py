@@ -419,3 +419,17 @@ def test_fidelity_of_an_image_far_off_the_object(far, axis):
     for a, b in zip(fused, _value_and_grads(fid, args)):
         assert torch.isfinite(torch.view_as_real(a) if a.is_complex() else a).all()
         assert rel_l2(a.cpu().numpy(), b.cpu().numpy()) < 1e-5
+
+
+@pytest.mark.parametrize("mag", [1e4, -1e7, 1e30, float("inf"), -float("inf")])
+def test_fidelity_of_an_image_magnified_off_the_object(mag):
+    """At a magnification that puts every pixel off the object, infinite included,
+    an image sees its zeros: fused against composed."""
+    fid, args = _small_fidelity()
+    args[3][2, 1] = mag
+    fused = _value_and_grads(fid, args)
+    assert fid._use_fused(*args, False)
+    fid._use_fused = lambda *a: False
+    for a, b in zip(fused, _value_and_grads(fid, args)):
+        assert torch.isfinite(torch.view_as_real(a) if a.is_complex() else a).all()
+        assert rel_l2(a.cpu().numpy(), b.cpu().numpy()) < 1e-5
