@@ -159,7 +159,7 @@ class _ChunkMisfit(torch.autograd.Function):
     @staticmethod
     @once_differentiable
     def backward(ctx, g):
-        x, prb, pos, mag, data = ctx.saved_tensors
+        x, prb, pos, mag, data = (t.contiguous() for t in ctx.saved_tensors)   # as a hook may not leave them
         cascade = ctx.cascade
         c = cascade.coeff(x)
         gc, gpos, gprb = torch.empty_like(c), torch.empty_like(pos), torch.empty_like(prb)

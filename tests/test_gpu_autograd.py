@@ -433,3 +433,20 @@ def test_fidelity_of_an_image_magnified_off_the_object(mag):
     for a, b in zip(fused, _value_and_grads(fid, args)):
         assert torch.isfinite(torch.view_as_real(a) if a.is_complex() else a).all()
         assert rel_l2(a.cpu().numpy(), b.cpu().numpy()) < 1e-5
+
+
+@pytest.mark.parametrize("proj", [False, True])
+def test_fidelity_under_saved_tensor_hooks(proj):
+    """Saved tensors kept on the host, and ones that come back with other strides:
+    the gradients without hooks, to the bit."""
+    fid, args = _small_fidelity(chunk=3)
+    if proj:
+        args[0] = torch.cat([t.R(args[0]) for t in fid.tomos])
+    ref = _value_and_grads(fid, args, proj)
+    strided = lambda t: torch.stack([t, t], -1)[..., 0]
+    for hooks in (torch.autograd.graph.save_on_cpu(pin_memory=True),
+                  torch.autograd.graph.saved_tensors_hooks(lambda t: t.cpu(), lambda t: strided(t.cuda()))):
+        with hooks:
+            got = _value_and_grads(fid, args, proj)
+        for a, b in zip(got, ref):
+            assert torch.equal(a, b)
